@@ -149,12 +149,14 @@ extern "C" int eg_host_free(void *p) {
     return EG_OK;
 }
 
+static void drop_scratch(eg_ctx *c);
 extern "C" int eg_close(eg_ctx *c) {
     if (!c) return EG_OK;
     if (c->live_graphs > 0) return eg_fail(EG_EINVAL, "eg_close: %d graphs are still open", c->live_graphs);
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaStreamSynchronize(c->copy_stream);
+    drop_scratch(c);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     for (cudaEvent_t e : c->evk) cudaEventDestroy(e);
@@ -175,12 +177,22 @@ extern "C" int eg_sync(eg_ctx *c) {
 extern "C" uint64_t eg_bytes_in_use(eg_ctx *c) { return c ? c->in_use : 0; }
 extern "C" uint64_t eg_kernel_launches(eg_ctx *c) { return c ? c->launches : 0; }
 
+// The context's scratch, beyond the buffers of its graphs.
+static void drop_scratch(eg_ctx *c) {
+    cudaStreamSynchronize(c->stream);
+    eg_buf_free(c, c->sort_ws);
+    eg_buf_free(c, c->scan_ws);
+}
+
 int eg_dmalloc(eg_ctx *c, void **p, uint64_t bytes) {
     *p = nullptr;
     if (bytes == 0) return EG_OK;
-    if (c->budget && c->in_use + bytes > c->budget)
-        return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
-                       (unsigned long long)c->in_use, (unsigned long long)bytes, (unsigned long long)c->budget);
+    if (c->budget && c->in_use + bytes > c->budget) {
+        drop_scratch(c);
+        if (c->in_use + bytes > c->budget)
+            return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
+                           (unsigned long long)c->in_use, (unsigned long long)bytes, (unsigned long long)c->budget);
+    }
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -501,32 +513,31 @@ __global__ void k_scan_apply(const uint32_t *in, uint64_t len, const uint32_t *o
 }
 }  // namespace
 
+// `sums`: room for the tile sums of this level and the ones above it.
+static int exscan_level(eg_ctx *ctx, const uint32_t *in, uint32_t *out, uint64_t len, uint32_t *sums) {
+    const uint32_t nb = eg_div_up(len, SCAN_TILE);
+    if (nb > 1) {
+        k_scan_reduce<<<nb, SCAN_T, 0, ctx->stream>>>(in, len, sums);
+        EG_LAUNCHED(ctx);
+        EG_TRY(exscan_level(ctx, sums, sums, nb, sums + nb + 1));  // in place: a block reads its tile before writing
+    }
+    k_scan_apply<<<nb, SCAN_T, 0, ctx->stream>>>(in, len, nb > 1 ? sums : nullptr, out, 1);
+    EG_LAUNCHED(ctx);
+    return EG_OK;
+}
+
 int eg_exscan_u32(eg_ctx *ctx, const uint32_t *in, uint32_t *out, uint64_t len) {
     if (len == 0) {
         EG_CUDA(cudaMemsetAsync(out, 0, sizeof(uint32_t), ctx->stream));
         return EG_OK;
     }
-    uint32_t nb = eg_div_up(len, SCAN_TILE);
-    if (nb == 1) {
-        k_scan_apply<<<1, SCAN_T, 0, ctx->stream>>>(in, len, nullptr, out, 1);
-        EG_LAUNCHED(ctx);
-        return EG_OK;
+    uint64_t words = 0;
+    for (uint64_t l = len; l > 1;) {
+        l = (l + SCAN_TILE - 1) / SCAN_TILE;
+        words += l + 1;
     }
-    uint32_t *sums = nullptr;
-    EG_TRY(eg_dmalloc(ctx, (void **)&sums, (uint64_t)(nb + 1) * sizeof(uint32_t)));
-    k_scan_reduce<<<nb, SCAN_T, 0, ctx->stream>>>(in, len, sums);
-    EG_LAUNCHED(ctx);
-    int rc = eg_exscan_u32(ctx, sums, sums, nb);  // in-place is safe: one block reads all before writing
-    if (rc == EG_OK) {
-        k_scan_apply<<<nb, SCAN_T, 0, ctx->stream>>>(in, len, sums, out, 1);
-        ctx->launches++;
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = eg_fail(EG_ECUDA, "scan apply: %s", cudaGetErrorString(e));
-    }
-    // free after the stream has consumed it
-    cudaStreamSynchronize(ctx->stream);
-    eg_dfree(ctx, sums, (uint64_t)(nb + 1) * sizeof(uint32_t));
-    return rc;
+    EG_TRY(eg_buf_ensure(ctx, ctx->scan_ws, words * 4 + 4));
+    return exscan_level(ctx, in, out, len, bp<uint32_t>(ctx->scan_ws));
 }
 
 // ============================================================== histogram
@@ -551,103 +562,358 @@ int eg_histogram(eg_ctx *ctx, const uint32_t *keys, uint64_t len, uint32_t *hist
 }
 
 // ============================================================== radix sort
-// Stable LSD radix sort, up to 8 bits per pass.  Per pass:
-//  1. k_rs_count: per-tile digit histogram -> counts[digit][tile]
-//  2. exclusive scan over counts (digit-major, tiles in order)
-//  3. k_rs_scatter: stable rank of every key inside its tile (warps take
-//     contiguous sub-tiles; __match_any_sync groups equal digits of a
-//     32-key chunk), staging through shared memory so the global writes are
-//     runs of consecutive addresses.
+// Stable LSD radix sort of (key, value) pairs, 8 bits per pass (9 where that
+// saves a pass).  Per pass:
+//  1. k_rs_count: digit histogram of each CTA's range of tiles -> counts[digit][CTA]
+//  2. k_rs_offs:  exclusive scan of each digit's row of counts, digit totals
+//  3. k_rs_scatter: the CTAs walk the same ranges tile by tile.  Stable rank of
+//     every key inside its tile (warps take contiguous sub-tiles; the lanes of
+//     a 32-key chunk with equal digits are found by one ballot per digit bit),
+//     staging through shared memory so that the global writes are runs of
+//     consecutive addresses; the CTA's next address per digit stays in shared
+//     memory from tile to tile.
+// Bound by HBM: 4 + 16 bytes per pair and pass.  One range of tiles per
+// resident CTA keeps the histogram at 2 * SMs words per digit (one word per
+// tile and digit had to be scanned through memory before), and the ballots
+// replace __match_any_sync, whose issue rate (one per ~43 cycles and SM)
+// bounded both kernels.  Pass over 134 M pairs (RMAT-22 undirected, 22-bit
+// keys): count 98 us (623 us before), scatter 681 us (942 us).
+// Measured at 134 M pairs, 256 threads x 16 pairs, 3 CTAs per SM: 681 us;
+// 512 x 16, 2: 712; 384 x 12, 3: 712; 256 x 12, 4: 739; 256 x 24, 2: 674
+// (larger tiles, fewer CTAs for small inputs); 256 x 8, 6: 955; 128 x 16, 6: 875.
+// The LSU pipe (the counters' and the staged pairs' bank conflicts) is the
+// busiest unit, HBM at 40 %.
 namespace {
-constexpr int RS_T = 256, RS_I = 16, RS_TILE = RS_T * RS_I, RS_W = RS_T / 32, RS_BINS = 256;
+constexpr int RS_T = 256, RS_I = 16, RS_TILE = RS_T * RS_I, RS_W = RS_T / 32;
+constexpr int RS_CTAS_PER_SM = 3;
 
-__global__ void __launch_bounds__(RS_T) k_rs_count(const uint32_t *keys, uint64_t len, int shift, uint32_t mask,
-                                                  uint32_t ntiles, uint32_t *counts) {
-    __shared__ uint32_t hist[RS_BINS];
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
-#pragma unroll 4
-    for (int i = 0; i < RS_I; i++) {
-        uint64_t idx = base + (uint64_t)i * RS_T + threadIdx.x;
-        bool valid = idx < len;
-        uint32_t d = valid ? (keys[idx] >> shift) & mask : 0xffffffffu;
-        uint32_t peers = __match_any_sync(EG_FULL_MASK, d);
-        if (valid && (eg_lanemask_lt() & peers) == 0) atomicAdd(&hist[d], __popc(peers));
+// Where a pass reads its keys and values: two arrays, or (the first pass of
+// the layout build) the input pairs in place, the reversed copies after them
+// when undirected, as preload_graph lays out memblock (init_all.c:81-110).
+struct RsArrays {
+    const uint32_t *k, *v;
+    __device__ __forceinline__ uint32_t key(uint64_t i) const { return __ldcs(k + i); }
+    __device__ __forceinline__ uint32_t value(uint64_t i) const { return __ldcs(v + i); }
+    __device__ __forceinline__ bool bad(uint64_t) const { return false; }
+    static constexpr bool checked = false;
+    // the words of entries [i, i + RS_TILE), entry i + j at [j * STRIDE]
+    static constexpr int STRIDE = 1;
+    __device__ __forceinline__ bool whole(uint64_t) const { return true; }
+    __device__ __forceinline__ const uint32_t *keys(uint64_t i) const { return k + i; }
+    __device__ __forceinline__ const uint32_t *values(uint64_t i) const { return v + i; }
+};
+struct RsPairs {
+    const uint2 *pairs;
+    uint64_t m_in;
+    uint32_t n;
+    __device__ __forceinline__ uint2 at(uint64_t i) const {
+        const uint2 p = __ldg(pairs + (i < m_in ? i : i - m_in));
+        return i < m_in ? p : make_uint2(p.y, p.x);
     }
+    __device__ __forceinline__ uint32_t key(uint64_t i) const { return at(i).x; }
+    __device__ __forceinline__ uint32_t value(uint64_t i) const { return at(i).y; }
+    __device__ __forceinline__ bool bad(uint64_t i) const {
+        const uint2 p = at(i);
+        return p.x >= n || p.y >= n;
+    }
+    static constexpr bool checked = true;
+    static constexpr int STRIDE = 2;
+    // whether the tile from entry i lies on one side of m_in
+    __device__ __forceinline__ bool whole(uint64_t i) const { return i >= m_in || i + RS_TILE <= m_in; }
+    __device__ __forceinline__ const uint32_t *keys(uint64_t i) const {
+        return reinterpret_cast<const uint32_t *>(pairs) + (i < m_in ? 2 * i : 2 * (i - m_in) + 1);
+    }
+    __device__ __forceinline__ const uint32_t *values(uint64_t i) const {
+        return reinterpret_cast<const uint32_t *>(pairs) + (i < m_in ? 2 * i + 1 : 2 * (i - m_in));
+    }
+};
+
+template <int BITS, class Src>
+__global__ void __launch_bounds__(RS_T) k_rs_count(const Src src, uint64_t len, int shift, uint32_t mask,
+                                                  uint32_t ntiles, uint32_t per, uint32_t *counts, uint32_t *bad) {
+    constexpr int BINS = 1 << BITS, COPIES = 4;  // copies: fewer warps meet on one word
+    __shared__ uint32_t hist[COPIES][BINS];
+    for (int i = threadIdx.x; i < COPIES * BINS; i += RS_T) (&hist[0][0])[i] = 0;
     __syncthreads();
-    if (threadIdx.x <= mask) counts[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = hist[threadIdx.x];
+    uint32_t *h = hist[(threadIdx.x >> 5) % COPIES];
+    const uint32_t t0 = blockIdx.x * per, t1 = t0 + per < ntiles ? t0 + per : ntiles;
+    bool anybad = false;
+    for (uint32_t t = t0; t < t1; t++) {
+        const uint64_t base = (uint64_t)t * RS_TILE + threadIdx.x;
+        if ((uint64_t)(t + 1) * RS_TILE <= len && src.whole((uint64_t)t * RS_TILE)) {
+            const uint32_t *kp = src.keys((uint64_t)t * RS_TILE) + threadIdx.x * Src::STRIDE;
+            uint32_t k[RS_I];
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) k[i] = __ldg(kp + i * RS_T * Src::STRIDE);
+            if constexpr (Src::checked) {
+                const uint32_t *vp = src.values((uint64_t)t * RS_TILE) + threadIdx.x * Src::STRIDE;
+#pragma unroll
+                for (int i = 0; i < RS_I; i++) anybad |= k[i] >= src.n || __ldg(vp + i * RS_T * Src::STRIDE) >= src.n;
+            }
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) atomicAdd(&h[(k[i] >> shift) & mask], 1u);
+        } else {
+            for (int i = 0; i < RS_I; i++) {
+                const uint64_t idx = base + (uint64_t)i * RS_T;
+                if (idx >= len) break;
+                atomicAdd(&h[(src.key(idx) >> shift) & mask], 1u);
+                if (Src::checked) anybad |= src.bad(idx);
+            }
+        }
+    }
+    if (Src::checked && __any_sync(EG_FULL_MASK, anybad) && (threadIdx.x & 31) == 0) atomicOr(bad, 1u);
+    __syncthreads();
+    for (uint32_t d = threadIdx.x; d <= mask; d += RS_T) {
+        uint32_t s = 0;
+#pragma unroll
+        for (int c = 0; c < COPIES; c++) s += hist[c][d];
+        counts[(uint64_t)d * gridDim.x + blockIdx.x] = s;
+    }
 }
 
-__global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
-                                                    uint32_t *vout, uint64_t len, int shift, uint32_t mask,
-                                                    uint32_t ntiles, const uint32_t *offs) {
-    __shared__ uint32_t wcnt[RS_W][RS_BINS];
-    __shared__ uint32_t loc[RS_BINS];
-    __shared__ uint32_t glob[RS_BINS];
+// One block per digit: its row of `b` counts becomes its exclusive scan.
+__global__ void __launch_bounds__(256) k_rs_offs(uint32_t *counts, uint32_t b, uint32_t *totals) {
     __shared__ uint32_t sh[33];
-    __shared__ uint32_t sk[RS_TILE];
-    __shared__ uint32_t sv[RS_TILE];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < RS_W * RS_BINS; i += RS_T) (&wcnt[0][0])[i] = 0;
-    __syncthreads();
-    const uint64_t tile0 = (uint64_t)blockIdx.x * RS_TILE;
-    const uint64_t base = tile0 + (uint64_t)warp * (RS_I * 32);
-    const uint32_t lt = eg_lanemask_lt();
-    uint32_t k[RS_I], v[RS_I], r[RS_I], dg[RS_I];
-#pragma unroll
-    for (int i = 0; i < RS_I; i++) {
-        uint64_t idx = base + (uint64_t)i * 32 + lane;
-        bool valid = idx < len;
-        k[i] = valid ? kin[idx] : 0u;
-        v[i] = valid ? vin[idx] : 0u;
-        dg[i] = valid ? (k[i] >> shift) & mask : (uint32_t)RS_BINS;
-    }
-#pragma unroll
-    for (int i = 0; i < RS_I; i++) {
-        uint32_t d = dg[i];
-        uint32_t peers = __match_any_sync(EG_FULL_MASK, d);
-        uint32_t below = __popc(peers & lt);
-        uint32_t cur = d < RS_BINS ? wcnt[warp][d] : 0u;
-        r[i] = cur + below;
-        __syncwarp();
-        if (d < RS_BINS && below == 0) wcnt[warp][d] = cur + __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    {
-        const int d = threadIdx.x;  // RS_T == RS_BINS
-        uint32_t run = 0;
-#pragma unroll
-        for (int w = 0; w < RS_W; w++) {
-            uint32_t c = wcnt[w][d];
-            wcnt[w][d] = run;
-            run += c;
-        }
+    uint32_t *row = counts + (uint64_t)blockIdx.x * b;
+    uint32_t run = 0;
+    for (uint32_t i0 = 0; i0 < b; i0 += 256) {
+        const uint32_t i = i0 + threadIdx.x;
         uint32_t ex;
-        block_exscan(run, ex, sh);
-        loc[d] = ex;
-        glob[d] = (uint32_t)d <= mask ? offs[(uint64_t)d * ntiles + blockIdx.x] : 0u;
+        const uint32_t tot = block_exscan(i < b ? row[i] : 0u, ex, sh);
+        if (i < b) row[i] = run + ex;
+        run += tot;
     }
-    __syncthreads();
+    if (threadIdx.x == 0) totals[blockIdx.x] = run;
+}
+
+// Lanes of the warp whose digit equals this lane's.
+template <int BITS>
+__device__ __forceinline__ uint32_t rs_match(uint32_t d, uint32_t peers) {
 #pragma unroll
-    for (int i = 0; i < RS_I; i++) {
-        uint32_t d = dg[i];
-        if (d < RS_BINS) {
-            uint32_t pos = loc[d] + wcnt[warp][d] + r[i];
-            sk[pos] = k[i];
-            sv[pos] = v[i];
+    for (int b = 0; b < BITS; b++) {
+        const bool bit = d & (1u << b);
+        const uint32_t v = __ballot_sync(EG_FULL_MASK, bit);
+        peers &= bit ? v : ~v;
+    }
+    return peers;
+}
+
+template <int BITS>
+struct RsSmem {
+    uint2 kv[RS_TILE];               // the tile's pairs in output order
+    uint32_t wcnt[RS_W][1 << BITS];  // a warp's keys of a digit, then its first place for them in kv
+    uint32_t glob[1 << BITS];  // the digit's next output place
+    uint32_t out[1 << BITS];   // output place of staged place 0, were it of this digit
+    uint32_t sh[33];
+};
+
+template <int BITS, class Src>
+__global__ void __launch_bounds__(RS_T, RS_CTAS_PER_SM) k_rs_scatter(const Src src, uint32_t *__restrict__ kout,
+                                                                     uint32_t *__restrict__ vout, uint64_t len,
+                                                                     int shift, uint32_t mask, uint32_t ntiles,
+                                                                     uint32_t per, const uint32_t *__restrict__ offs,
+                                                                     const uint32_t *__restrict__ totals) {
+    constexpr int BINS = 1 << BITS, DPT = BINS > RS_T ? BINS / RS_T : 1;  // digits per thread
+    extern __shared__ __align__(16) unsigned char rs_raw[];
+    RsSmem<BITS> &sm = *reinterpret_cast<RsSmem<BITS> *>(rs_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt = eg_lanemask_lt();
+    const uint32_t d0 = threadIdx.x * DPT;  // this thread's digits [d0, d0 + DPT), when below BINS
+    {
+        uint32_t tot[DPT], s = 0, ex;
+#pragma unroll
+        for (int j = 0; j < DPT; j++) {
+            tot[j] = d0 + j <= mask ? totals[d0 + j] : 0u;
+            s += tot[j];
+        }
+        block_exscan(s, ex, sm.sh);
+#pragma unroll
+        for (int j = 0; j < DPT; j++) {
+            if (d0 + j <= mask) sm.glob[d0 + j] = ex + offs[(uint64_t)(d0 + j) * gridDim.x + blockIdx.x];
+            ex += tot[j];
         }
     }
+    for (int i = threadIdx.x; i < RS_W * BINS / 4; i += RS_T)
+        reinterpret_cast<uint4 *>(&sm.wcnt[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t t0 = blockIdx.x * per, t1 = t0 + per < ntiles ? t0 + per : ntiles;
+    uint32_t *wc = sm.wcnt[warp];
+    const uint32_t woff = warp * (RS_I * 32) + lane;  // the thread's entries: woff + 32 * i
+    uint32_t k[RS_I];
+    // whole tiles need no bounds and have one base address
+    auto whole = [&](uint32_t t) { return (uint64_t)(t + 1) * RS_TILE <= len && src.whole((uint64_t)t * RS_TILE); };
+    auto load_keys = [&](uint32_t t) {
+        if (whole(t)) {
+            const uint32_t *kp = src.keys((uint64_t)t * RS_TILE) + woff * Src::STRIDE;
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) k[i] = __ldg(kp + i * 32 * Src::STRIDE);
+        } else {
+            const uint64_t base = (uint64_t)t * RS_TILE + woff;
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) k[i] = base + i * 32 < len ? src.key(base + i * 32) : 0u;
+        }
+    };
+    if (t0 < t1) load_keys(t0);
     __syncthreads();
-    const uint32_t valid_count = (uint32_t)((len - tile0) < (uint64_t)RS_TILE ? (len - tile0) : (uint64_t)RS_TILE);
-    for (uint32_t s = threadIdx.x; s < valid_count; s += RS_T) {
-        uint32_t key = sk[s];
-        uint32_t d = (key >> shift) & mask;
-        uint32_t gpos = glob[d] + (s - loc[d]);
-        kout[gpos] = key;
-        vout[gpos] = sv[s];
+    for (uint32_t t = t0; t < t1; t++) {
+        const uint64_t tile0 = (uint64_t)t * RS_TILE;
+        const uint64_t base = tile0 + woff;
+        const bool full = whole(t);
+        uint32_t r[RS_I], v[RS_I];  // the values are in flight while the digits' places are worked out
+        if (full) {
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) {
+                const uint32_t d = (k[i] >> shift) & mask;
+                const uint32_t peers = rs_match<BITS>(d, EG_FULL_MASK);
+                const uint32_t below = __popc(peers & lt);
+                const uint32_t cur = wc[d];
+                r[i] = cur + below;
+                __syncwarp();
+                if (below == 0) wc[d] = cur + __popc(peers);
+                __syncwarp();
+            }
+            const uint32_t *vp = src.values(tile0) + woff * Src::STRIDE;
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) v[i] = __ldg(vp + i * 32 * Src::STRIDE);
+        } else {
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) {
+                const bool valid = base + i * 32 < len;
+                const uint32_t d = (k[i] >> shift) & mask;
+                const uint32_t peers = rs_match<BITS>(d, __ballot_sync(EG_FULL_MASK, valid));
+                const uint32_t below = __popc(peers & lt);
+                const uint32_t cur = wc[d];
+                r[i] = cur + below;
+                __syncwarp();
+                if (valid && below == 0) wc[d] = cur + __popc(peers);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int i = 0; i < RS_I; i++) v[i] = base + i * 32 < len ? src.value(base + i * 32) : 0u;
+        }
+        __syncthreads();
+        {
+            uint32_t run[DPT], s = 0, ex;
+#pragma unroll
+            for (int j = 0; j < DPT; j++) {
+                run[j] = 0;
+                if (d0 + j < BINS) {
+#pragma unroll
+                    for (int w = 0; w < RS_W; w++) run[j] += sm.wcnt[w][d0 + j];
+                }
+                s += run[j];
+            }
+            block_exscan(s, ex, sm.sh);
+#pragma unroll
+            for (int j = 0; j < DPT; j++) {
+                if (d0 + j < BINS) {
+                    const uint32_t g = sm.glob[d0 + j];
+                    sm.out[d0 + j] = g - ex;
+                    sm.glob[d0 + j] = g + run[j];
+#pragma unroll
+                    for (int w = 0; w < RS_W; w++) {
+                        const uint32_t c = sm.wcnt[w][d0 + j];
+                        sm.wcnt[w][d0 + j] = ex;
+                        ex += c;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < RS_I; i++) {
+            if (base + i * 32 < len) sm.kv[wc[(k[i] >> shift) & mask] + r[i]] = make_uint2(k[i], v[i]);
+        }
+        __syncthreads();
+        if (t + 1 < t1) load_keys(t + 1);  // in flight while this tile is written out
+        const uint32_t cnt = len - tile0 < RS_TILE ? (uint32_t)(len - tile0) : (uint32_t)RS_TILE;
+#pragma unroll 4
+        for (uint32_t s = threadIdx.x; s < cnt; s += RS_T) {
+            const uint2 x = sm.kv[s];
+            const uint32_t g = sm.out[(x.x >> shift) & mask] + s;
+            kout[g] = x.x;
+            vout[g] = x.y;
+        }
+        for (int i = threadIdx.x; i < RS_W * BINS / 4; i += RS_T)
+            reinterpret_cast<uint4 *>(&sm.wcnt[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
     }
+}
+
+// Digit width of a sort by `bits` bits: 8, or 9 where that saves a pass
+// (9..., 17-18, 25-27 bits: a pass costs 20 bytes per pair, twice the bins
+// only shorter runs).
+int rs_width(int bits) {
+    const int p8 = (bits + 7) / 8, p9 = (bits + 8) / 9;
+    return p9 < p8 ? 9 : 8;
+}
+struct RsPlan {
+    uint32_t ntiles, per, ctas;
+};
+RsPlan rs_plan(eg_ctx *ctx, uint64_t len) {
+    RsPlan p;
+    p.ntiles = eg_div_up(len, RS_TILE);
+    const uint32_t cap = (uint32_t)ctx->sm_count * RS_CTAS_PER_SM;
+    p.per = eg_div_up(p.ntiles, cap);
+    p.ctas = eg_div_up(p.ntiles, p.per);
+    return p;
+}
+uint64_t rs_ws_bytes(eg_ctx *ctx, uint64_t len, int bits) {
+    return (((uint64_t)rs_plan(ctx, len).ctas + 1) << rs_width(bits)) * sizeof(uint32_t);
+}
+
+// One pass by the `pb` key bits from `shift`.  ws: rs_ws_bytes.  bad
+// (RsPairs): set when an endpoint is out of range; `*host_bad` is then read
+// before the scatter and nothing is written.
+template <int BITS, class Src>
+int rs_pass(eg_ctx *ctx, const Src &src, uint32_t *kout, uint32_t *vout, uint64_t len, int shift, int pb, uint32_t *ws,
+            uint32_t *bad, bool *any_bad) {
+    const RsPlan p = rs_plan(ctx, len);
+    const uint32_t mask = (1u << pb) - 1u;
+    uint32_t *counts = ws, *totals = ws + ((uint64_t)p.ctas << BITS);
+    constexpr size_t smem = sizeof(RsSmem<BITS>);
+    EG_CUDA(cudaFuncSetAttribute(k_rs_scatter<BITS, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_rs_count<BITS, Src><<<p.ctas, RS_T, 0, ctx->stream>>>(src, len, shift, mask, p.ntiles, p.per, counts, bad);
+    EG_LAUNCHED(ctx);
+    if (Src::checked && bad) {
+        uint32_t *h = (uint32_t *)ctx->h_pinned;
+        EG_TRY(eg_readback_wait(ctx, h, bad, 4, ctx->stream));
+        *any_bad = *h != 0;
+        if (*any_bad) return EG_OK;
+    }
+    k_rs_offs<<<mask + 1, 256, 0, ctx->stream>>>(counts, p.ctas, totals);
+    EG_LAUNCHED(ctx);
+    k_rs_scatter<BITS, Src><<<p.ctas, RS_T, smem, ctx->stream>>>(src, kout, vout, len, shift, mask, p.ntiles, p.per,
+                                                                 counts, totals);
+    EG_LAUNCHED(ctx);
+    return EG_OK;
+}
+template <class Src>
+int rs_pass_w(eg_ctx *ctx, int width, const Src &src, uint32_t *kout, uint32_t *vout, uint64_t len, int shift, int pb,
+              uint32_t *ws, uint32_t *bad, bool *any_bad) {
+    return width == 9 ? rs_pass<9, Src>(ctx, src, kout, vout, len, shift, pb, ws, bad, any_bad)
+                      : rs_pass<8, Src>(ctx, src, kout, vout, len, shift, pb, ws, bad, any_bad);
+}
+
+// The sort from `src` (read only by the first pass) into (kd, vd), with the
+// pair (kt, vt) as the other buffer of the passes: it is not read when one
+// pass is enough.
+template <class Src>
+int rs_sort_into(eg_ctx *ctx, const Src &src, uint32_t *kd, uint32_t *vd, uint32_t *kt, uint32_t *vt, uint64_t len,
+                 int bits, uint32_t *ws, uint32_t *bad, bool *any_bad) {
+    const int width = rs_width(bits), passes = (bits + width - 1) / width, per = (bits + passes - 1) / passes;
+    for (int p = 0; p < passes; p++) {
+        const int shift = p * per, pb = bits - shift < per ? bits - shift : per;
+        const bool to_dest = ((passes - 1 - p) & 1) == 0;
+        uint32_t *ko = to_dest ? kd : kt, *vo = to_dest ? vd : vt;
+        if (p == 0) {
+            EG_TRY(rs_pass_w(ctx, width, src, ko, vo, len, shift, pb, ws, bad, any_bad));
+            if (any_bad && *any_bad) return EG_OK;
+        } else {
+            const RsArrays a{to_dest ? kt : kd, to_dest ? vt : vd};
+            EG_TRY(rs_pass_w(ctx, width, a, ko, vo, len, shift, pb, ws, nullptr, nullptr));
+        }
+    }
+    return EG_OK;
 }
 }  // namespace
 
@@ -656,63 +922,19 @@ int eg_radix_sort(eg_ctx *ctx, uint32_t *k_in, uint32_t *v_in, uint32_t *k_tmp, 
     *k_out = k_in;
     *v_out = v_in;
     if (len <= 1 || bits <= 0) return EG_OK;
-    int passes = (bits + 7) / 8;
-    int per = (bits + passes - 1) / passes;
-    uint32_t ntiles = eg_div_up(len, RS_TILE);
-    uint64_t ncount = (uint64_t)ntiles << per;
-    uint32_t *counts = nullptr, *offs = nullptr;
-    EG_TRY(eg_dmalloc(ctx, (void **)&counts, ncount * sizeof(uint32_t)));
-    int rc = eg_dmalloc(ctx, (void **)&offs, (ncount + 1) * sizeof(uint32_t));
-    if (rc != EG_OK) {
-        eg_dfree(ctx, counts, ncount * sizeof(uint32_t));
-        return rc;
-    }
-    uint32_t *ka = k_in, *va = v_in, *kb = k_tmp, *vb = v_tmp;
-    for (int p = 0; p < passes && rc == EG_OK; p++) {
-        int shift = p * per;
-        int pb = bits - shift < per ? bits - shift : per;
-        uint32_t mask = (1u << pb) - 1u;
-        uint64_t nc = (uint64_t)ntiles * (mask + 1);
-        k_rs_count<<<ntiles, RS_T, 0, ctx->stream>>>(ka, len, shift, mask, ntiles, counts);
-        ctx->launches++;
-        rc = eg_exscan_u32(ctx, counts, offs, nc);
-        if (rc != EG_OK) break;
-        k_rs_scatter<<<ntiles, RS_T, 0, ctx->stream>>>(ka, va, kb, vb, len, shift, mask, ntiles, offs);
-        ctx->launches++;
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = eg_fail(EG_ECUDA, "radix pass: %s", cudaGetErrorString(e));
-        uint32_t *t = ka; ka = kb; kb = t;
-        t = va; va = vb; vb = t;
-    }
-    cudaStreamSynchronize(ctx->stream);
-    eg_dfree(ctx, counts, ncount * sizeof(uint32_t));
-    eg_dfree(ctx, offs, (ncount + 1) * sizeof(uint32_t));
-    *k_out = ka;
-    *v_out = va;
+    const int width = rs_width(bits), passes = (bits + width - 1) / width;
+    EG_TRY(eg_buf_ensure(ctx, ctx->sort_ws, rs_ws_bytes(ctx, len, bits)));
+    uint32_t *ws = bp<uint32_t>(ctx->sort_ws);
+    // the input pair is the first pass's source and the passes' second buffer
+    uint32_t *kd = passes & 1 ? k_tmp : k_in, *vd = passes & 1 ? v_tmp : v_in;
+    uint32_t *kt = passes & 1 ? k_in : k_tmp, *vt = passes & 1 ? v_in : v_tmp;
+    const int rc = rs_sort_into(ctx, RsArrays{k_in, v_in}, kd, vd, kt, vt, len, bits, ws, nullptr, nullptr);
+    *k_out = kd;
+    *v_out = vd;
     return rc;
 }
 
 // ============================================================== builders
-// Unpacks the input pairs into (key, value) arrays: the file's edges in file
-// order, then (undirected) the reversed copies, as preload_graph lays out
-// memblock (init_all.c:81-110).  by_src selects key=src,value=dst.
-__global__ void k_unpack(const uint32_t *pairs, uint64_t m_in, int undirected, uint32_t n, uint32_t *keys,
-                         uint32_t *vals, uint32_t *bad) {
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t M = undirected ? 2 * m_in : m_in;
-    uint32_t anybad = 0;
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < M; k += stride) {
-        uint64_t e = k < m_in ? k : k - m_in;
-        uint2 p = reinterpret_cast<const uint2 *>(pairs)[e];
-        uint32_t s = k < m_in ? p.x : p.y;
-        uint32_t d = k < m_in ? p.y : p.x;
-        anybad |= (s >= n) | (d >= n);
-        keys[k] = s;
-        vals[k] = d;
-    }
-    if (__any_sync(EG_FULL_MASK, anybad) && (threadIdx.x & 31) == 0) atomicOr(bad, 1u);
-}
-
 static int bits_for(uint32_t n) {
     if (n <= 1) return 1;
     uint32_t x = n - 1;
@@ -721,20 +943,67 @@ static int bits_for(uint32_t n) {
     return b;
 }
 
+// First and one-past-last place of every row's run in the sorted row ids
+// (both arrays zeroed: rows without entries keep 0, 0).  Four entries per
+// thread; 4 bytes per entry.
+__global__ void __launch_bounds__(256) k_row_runs(const uint32_t *__restrict__ rid, uint32_t m, uint32_t *first,
+                                                  uint32_t *last) {
+    const uint32_t nq = (uint32_t)(((uint64_t)m + 3) >> 2);
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        const uint32_t b = q * 4;
+        uint32_t prev = b ? __ldg(rid + b - 1) : 0u;
+        uint4 x;
+        if (b + 4 <= m) x = __ldg(reinterpret_cast<const uint4 *>(rid) + q);
+        else {
+            x.x = __ldg(rid + b);
+            x.y = b + 1 < m ? __ldg(rid + b + 1) : 0u;
+            x.z = b + 2 < m ? __ldg(rid + b + 2) : 0u;
+            x.w = 0u;
+        }
+        const uint32_t r[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (b + i >= m) break;
+            if (b + i == 0 || r[i] != prev) {
+                first[r[i]] = b + i;
+                if (b + i) last[prev] = b + i;
+            }
+            prev = r[i];
+        }
+        if (b + 4 >= m) last[prev] = m;
+    }
+}
+__global__ void k_run_lengths(const uint32_t *__restrict__ first, uint32_t n, uint32_t *last_to_len) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        last_to_len[v] -= first[v];
+}
+
+// Degrees and row pointers of an adjacency from its sorted row ids.
+static int rows_from_rid(eg_ctx *ctx, const uint32_t *rid, uint64_t M, uint32_t n, uint32_t *deg, uint32_t *ptr) {
+    EG_CUDA(cudaMemsetAsync(deg, 0, (uint64_t)n * 4, ctx->stream));
+    if (M) {
+        EG_CUDA(cudaMemsetAsync(ptr, 0, (uint64_t)n * 4, ctx->stream));  // the runs' starts until the scan
+        k_row_runs<<<grid_for(ctx, (M + 3) / 4), 256, 0, ctx->stream>>>(rid, (uint32_t)M, ptr, deg);
+        EG_LAUNCHED(ctx);
+        k_run_lengths<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(ptr, n, deg);
+        EG_LAUNCHED(ctx);
+    }
+    return eg_exscan_u32(ctx, deg, ptr, n);
+}
+
+// CSR (and CSC) of the input pairs: the first pass of the CSR's sort reads
+// the pairs where they lie, the last pass of each sort writes the adjacency's
+// own arrays, and one more pair of arrays serves the passes in between.
 static int build_adj_pair(eg_graph *g, bool want_csc) {
     eg_ctx *ctx = g->ctx;
     const uint64_t M = g->m;
     const uint32_t n = g->n;
-    eg_buf ka, va, kb, vb;
+    eg_buf ka, va;
     int rc = EG_OK;
-    uint32_t *ks = nullptr, *vs = nullptr;
-    uint32_t *hbad = (uint32_t *)ctx->h_pinned;
     auto cleanup = [&]() {
         cudaStreamSynchronize(ctx->stream);
         eg_buf_free(ctx, ka);
         eg_buf_free(ctx, va);
-        eg_buf_free(ctx, kb);
-        eg_buf_free(ctx, vb);
     };
 #define BTRY(x)                 \
     do {                        \
@@ -744,57 +1013,43 @@ static int build_adj_pair(eg_graph *g, bool want_csc) {
             return rc;          \
         }                       \
     } while (0)
+    const int bits = bits_for(n);
     BTRY(eg_buf_ensure(ctx, ka, (M + 1) * 4));
     BTRY(eg_buf_ensure(ctx, va, (M + 1) * 4));
-    BTRY(eg_buf_ensure(ctx, kb, (M + 1) * 4));
-    BTRY(eg_buf_ensure(ctx, vb, (M + 1) * 4));
-    uint32_t *dbad = bp<uint32_t>(kb) + M;  // one spare word past the data
-    if (cudaMemsetAsync(dbad, 0, 4, ctx->stream) != cudaSuccess) BTRY(eg_fail(EG_ECUDA, "memset"));
-    if (M) {
-        k_unpack<<<grid_for(ctx, M), 256, 0, ctx->stream>>>(bp<uint32_t>(g->pairs), g->m_in, (g->flags & EG_UNDIRECTED) != 0, n,
-                                                           bp<uint32_t>(ka), bp<uint32_t>(va), dbad);
-        ctx->launches++;
-    }
-    if (cudaMemcpyAsync(hbad, dbad, 4, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-        BTRY(eg_fail(EG_ECUDA, "unpack: %s", cudaGetErrorString(cudaGetLastError())));
-    if (*hbad) BTRY(eg_fail(EG_ERANGE, "an edge endpoint is >= n=%u", n));
-    int bits = bits_for(n);
-    // CSR: stable sort by src, value dst
-    BTRY(eg_radix_sort(ctx, bp<uint32_t>(ka), bp<uint32_t>(va), bp<uint32_t>(kb), bp<uint32_t>(vb), M, bits, &ks, &vs));
+    uint32_t *dbad = bp<uint32_t>(ka) + M;  // the spare word
     BTRY(eg_buf_ensure(ctx, g->out_deg, (uint64_t)n * 4));
     BTRY(eg_buf_ensure(ctx, g->csr.ptr, ((uint64_t)n + 1) * 4));
     BTRY(eg_buf_ensure(ctx, g->csr.col, M * 4 + 16));
-    if (cudaMemsetAsync(g->out_deg.p, 0, (uint64_t)n * 4, ctx->stream) != cudaSuccess) BTRY(eg_fail(EG_ECUDA, "memset"));
-    BTRY(eg_histogram(ctx, ks, M, bp<uint32_t>(g->out_deg)));
-    BTRY(eg_exscan_u32(ctx, bp<uint32_t>(g->out_deg), bp<uint32_t>(g->csr.ptr), n));
-    if (M && cudaMemcpyAsync(g->csr.col.p, vs, M * 4, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-        BTRY(eg_fail(EG_ECUDA, "copy col"));
     BTRY(eg_buf_ensure(ctx, g->csr.rid, M * 4 + 16));
-    if (M && cudaMemcpyAsync(g->csr.rid.p, ks, M * 4, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-        BTRY(eg_fail(EG_ECUDA, "copy rid"));
+    if (want_csc) {
+        BTRY(eg_buf_ensure(ctx, g->in_deg, (uint64_t)n * 4));
+        BTRY(eg_buf_ensure(ctx, g->csc.ptr, ((uint64_t)n + 1) * 4));
+        BTRY(eg_buf_ensure(ctx, g->csc.col, M * 4 + 16));
+        BTRY(eg_buf_ensure(ctx, g->csc.rid, M * 4 + 16));
+    }
+    BTRY(eg_zero(ctx, dbad, 4, ctx->stream));
+    // CSR: stable sort by src, value dst
+    if (M) {
+        const RsPairs src{reinterpret_cast<const uint2 *>(g->pairs.p), g->m_in, n};
+        bool any_bad = false;
+        BTRY(eg_buf_ensure(ctx, ctx->sort_ws, rs_ws_bytes(ctx, M, bits)));
+        BTRY(rs_sort_into(ctx, src, bp<uint32_t>(g->csr.rid), bp<uint32_t>(g->csr.col), bp<uint32_t>(ka),
+                          bp<uint32_t>(va), M, bits, bp<uint32_t>(ctx->sort_ws), dbad, &any_bad));
+        if (any_bad) BTRY(eg_fail(EG_ERANGE, "an edge endpoint is >= n=%u", n));
+    }
+    BTRY(rows_from_rid(ctx, bp<uint32_t>(g->csr.rid), M, n, bp<uint32_t>(g->out_deg), bp<uint32_t>(g->csr.ptr)));
     g->built |= EG_LAYOUT_CSR;
     g->first_in_src = nullptr;
     g->wcc_list_src = nullptr;
     if (want_csc) {
-        // CSC: stable sort of the CSR entries by dst, value src.  The sorted
-        // src keys become the values; the CSR cols (a copy) become the keys.
-        // The temporaries are the buffer pair that does not hold the result.
-        uint32_t *k2 = vs, *v2 = ks;
-        uint32_t *kt = (ks == bp<uint32_t>(ka)) ? bp<uint32_t>(kb) : bp<uint32_t>(ka);
-        uint32_t *vt = (ks == bp<uint32_t>(ka)) ? bp<uint32_t>(vb) : bp<uint32_t>(va);
-        BTRY(eg_radix_sort(ctx, k2, v2, kt, vt, M, bits, &ks, &vs));
-        BTRY(eg_buf_ensure(ctx, g->in_deg, (uint64_t)n * 4));
-        BTRY(eg_buf_ensure(ctx, g->csc.ptr, ((uint64_t)n + 1) * 4));
-        BTRY(eg_buf_ensure(ctx, g->csc.col, M * 4 + 16));
-        if (cudaMemsetAsync(g->in_deg.p, 0, (uint64_t)n * 4, ctx->stream) != cudaSuccess) BTRY(eg_fail(EG_ECUDA, "memset"));
-        BTRY(eg_histogram(ctx, ks, M, bp<uint32_t>(g->in_deg)));
-        BTRY(eg_exscan_u32(ctx, bp<uint32_t>(g->in_deg), bp<uint32_t>(g->csc.ptr), n));
-        if (M && cudaMemcpyAsync(g->csc.col.p, vs, M * 4, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-            BTRY(eg_fail(EG_ECUDA, "copy col"));
-        BTRY(eg_buf_ensure(ctx, g->csc.rid, M * 4 + 16));
-        if (M && cudaMemcpyAsync(g->csc.rid.p, ks, M * 4, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-            BTRY(eg_fail(EG_ECUDA, "copy rid"));
+        // CSC: stable sort of the CSR entries by dst, value src
+        if (M) {
+            BTRY(eg_buf_ensure(ctx, ctx->sort_ws, rs_ws_bytes(ctx, M, bits)));  // a full budget may have dropped it
+            BTRY(rs_sort_into(ctx, RsArrays{bp<uint32_t>(g->csr.col), bp<uint32_t>(g->csr.rid)},
+                              bp<uint32_t>(g->csc.rid), bp<uint32_t>(g->csc.col), bp<uint32_t>(ka), bp<uint32_t>(va), M,
+                              bits, bp<uint32_t>(ctx->sort_ws), nullptr, nullptr));
+        }
+        BTRY(rows_from_rid(ctx, bp<uint32_t>(g->csc.rid), M, n, bp<uint32_t>(g->in_deg), bp<uint32_t>(g->csc.ptr)));
         g->built |= EG_LAYOUT_CSC;
         g->first_in_src = nullptr;
         g->wcc_list_src = nullptr;

@@ -41,6 +41,11 @@ void eg_clear_error();
 #define EG_KEV 8        // kernel launches timed individually per call
 #define EG_OUT_SLOTS 4  // device output slots of eg_bfs_batch (copy-out pipeline depth)
 #define EG_SB_MAX 64    // source blocks of the blocked CSC at most
+// A device buffer tracked against the context budget.
+struct eg_buf {
+    void *p = nullptr;
+    uint64_t bytes = 0;
+};
 struct eg_ctx {
     int device;
     int sm_count;
@@ -56,6 +61,7 @@ struct eg_ctx {
     cudaStream_t copy_stream;     // device-to-host copies overlapped with the next traversal
     cudaEvent_t ev_out[2 * EG_OUT_SLOTS];  // [slot]: outputs ready, [EG_OUT_SLOTS + slot]: copied out
     uint32_t rb_seq = 0;                   // eg_readback_wait: the last flag value asked for
+    eg_buf sort_ws, scan_ws;  // radix sort counts, scan sums: used on `stream` only, kept between calls
 };
 // eg_readback_wait's flag word: the last 64 bytes of the pinned staging area
 #define EG_RB_FLAG_OFF ((1u << 20) - 64u)
@@ -63,11 +69,6 @@ struct eg_ctx {
 int eg_dmalloc(eg_ctx *ctx, void **p, uint64_t bytes);
 void eg_dfree(eg_ctx *ctx, void *p, uint64_t bytes);
 
-// A device buffer tracked against the context budget.
-struct eg_buf {
-    void *p = nullptr;
-    uint64_t bytes = 0;
-};
 int eg_buf_ensure(eg_ctx *ctx, eg_buf &b, uint64_t bytes);  // grows (contents lost)
 // Small device-to-host readback into ctx->h_pinned (host_dst lies in it) by a
 // one-warp kernel on `st` instead of a copy engine, so that it does not queue
