@@ -177,35 +177,94 @@ extern "C" int eg_sync(eg_ctx *c) {
 extern "C" uint64_t eg_bytes_in_use(eg_ctx *c) { return c ? c->in_use : 0; }
 extern "C" uint64_t eg_kernel_launches(eg_ctx *c) { return c ? c->launches : 0; }
 
-// The context's scratch, beyond the buffers of its graphs.
+// ---- device memory
+// Blocks that are given back are kept for the context's next allocations, up
+// to EG_KEEP_BYTES of them, oldest given back to the driver first: a layout
+// build allocates and frees about 30 bytes per entry, and cudaMalloc and
+// cudaFree of 512 MB take 156 and 282 us here (2 GB: 0.6 and 1.0 ms).  Build
+// of undirected RMAT-22 from device pairs: 9.6 ms without, 5.5 ms with
+// kept blocks.  Kept blocks
+// never make an allocation fail: they go back to the driver when the budget
+// or the device has no room beside them, and with the context.
+#define EG_KEEP_BYTES (8ull << 30)
+#define EG_KEEP_BLOCKS 64u
+#define EG_KEEP_MIN 65536ull  // smaller blocks go straight back
+
+static void drop_kept(eg_ctx *c, uint64_t down_to) {
+    size_t k = 0;
+    while (k < c->kept.size() && c->kept_bytes > down_to) {
+        cudaFree(c->kept[k].p);  // waits for the device
+        c->kept_bytes -= c->kept[k].bytes;
+        k++;
+    }
+    c->kept.erase(c->kept.begin(), c->kept.begin() + k);
+}
+
+// Everything the context holds beyond the live buffers of its graphs.
 static void drop_scratch(eg_ctx *c) {
     cudaStreamSynchronize(c->stream);
     eg_buf_free(c, c->sort_ws);
     eg_buf_free(c, c->scan_ws);
+    drop_kept(c, 0);
 }
 
 int eg_dmalloc(eg_ctx *c, void **p, uint64_t bytes) {
     *p = nullptr;
     if (bytes == 0) return EG_OK;
-    if (c->budget && c->in_use + bytes > c->budget) {
+    if (c->budget && c->in_use + c->kept_bytes + bytes > c->budget) {
         drop_scratch(c);
         if (c->in_use + bytes > c->budget)
             return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
                            (unsigned long long)c->in_use, (unsigned long long)bytes, (unsigned long long)c->budget);
     }
+    // the smallest kept block that fits with at most an eighth to spare
+    size_t best = c->kept.size();
+    for (size_t i = 0; i < c->kept.size(); i++) {
+        const uint64_t b = c->kept[i].bytes;
+        if (b >= bytes && b <= bytes + bytes / 8 && (best == c->kept.size() || b < c->kept[best].bytes)) best = i;
+    }
+    if (best < c->kept.size()) {
+        if (c->kept_busy) {  // as after cudaFree: nothing queued anywhere still uses it
+            EG_CUDA(cudaDeviceSynchronize());
+            c->kept_busy = false;
+        }
+        *p = c->kept[best].p;
+        c->kept_bytes -= c->kept[best].bytes;
+        c->live[*p] = c->kept[best].bytes;
+        c->kept.erase(c->kept.begin() + best);
+        c->in_use += bytes;
+        return EG_OK;
+    }
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && (c->kept_bytes || c->sort_ws.p || c->scan_ws.p)) {
+        cudaGetLastError();
+        drop_scratch(c);
+        e = cudaMalloc(p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
         return eg_fail(EG_ENOMEM, "cudaMalloc(%llu): %s", (unsigned long long)bytes, cudaGetErrorString(e));
     }
+    c->live[*p] = bytes;
     c->in_use += bytes;
     return EG_OK;
 }
 void eg_dfree(eg_ctx *c, void *p, uint64_t bytes) {
     if (!p) return;
-    cudaFree(p);
     c->in_use -= bytes;
+    const auto it = c->live.find(p);
+    const uint64_t size = it == c->live.end() ? 0 : it->second;
+    if (it != c->live.end()) c->live.erase(it);
+    if (size < EG_KEEP_MIN || size > EG_KEEP_BYTES) {
+        cudaFree(p);
+        return;
+    }
+    drop_kept(c, EG_KEEP_BYTES - size);
+    if (c->kept.size() >= EG_KEEP_BLOCKS) drop_kept(c, c->kept_bytes - c->kept[0].bytes);
+    c->kept.push_back({p, size});
+    c->kept_bytes += size;
+    c->kept_busy = true;
 }
 int eg_buf_ensure(eg_ctx *c, eg_buf &b, uint64_t bytes) {
     if (b.bytes >= bytes && b.p) return EG_OK;

@@ -5,6 +5,9 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <unordered_map>
+#include <vector>
+
 #include "eg_gpu.h"
 
 #define EG_FULL_MASK 0xffffffffu
@@ -46,6 +49,11 @@ struct eg_buf {
     void *p = nullptr;
     uint64_t bytes = 0;
 };
+// A device block given back to the context and kept for its next allocation.
+struct eg_block {
+    void *p;
+    uint64_t bytes;
+};
 struct eg_ctx {
     int device;
     int sm_count;
@@ -61,6 +69,13 @@ struct eg_ctx {
     cudaStream_t copy_stream;     // device-to-host copies overlapped with the next traversal
     cudaEvent_t ev_out[2 * EG_OUT_SLOTS];  // [slot]: outputs ready, [EG_OUT_SLOTS + slot]: copied out
     uint32_t rb_seq = 0;                   // eg_readback_wait: the last flag value asked for
+    // eg_dmalloc's kept blocks, oldest first (their bytes are not in in_use),
+    // whether one of them may still be in use by work queued before it was
+    // given back, and the sizes of the live blocks
+    std::vector<eg_block> kept;
+    uint64_t kept_bytes = 0;
+    bool kept_busy = false;
+    std::unordered_map<void *, uint64_t> live;
     eg_buf sort_ws, scan_ws;  // radix sort counts, scan sums: used on `stream` only, kept between calls
 };
 // eg_readback_wait's flag word: the last 64 bytes of the pinned staging area

@@ -62,3 +62,29 @@ def test_bad_endpoint_is_refused(m):
         assert g.info().layouts == 0
         g.free()
     ctx.close()
+
+
+def test_kept_blocks_are_reused_and_given_back():
+    """Freed blocks serve the next graph, are not counted as in use, and give
+    way when the budget has no room beside them."""
+    import everythinggraph_gb300 as eg
+
+    ctx = eg.Context(0)
+    ref = None
+    for _ in range(3):  # the second and third graph are built in kept blocks
+        g = ctx.rmat(16, 1 << 20, 5, undirected=True).build(eg.CSR | eg.CSC)
+        got = g.adj(eg.CSC)
+        ref = ref or (got, ctx.bytes_in_use)
+        assert np.array_equal(got[0], ref[0][0]) and np.array_equal(got[1], ref[0][1])
+        assert ctx.bytes_in_use == ref[1]
+        lv, _ = g.bfs(int(g.sample_roots(1, 1)[0]))
+        assert lv.max() > 1
+        g.free()
+    ctx.close()
+    # the first graph's blocks (about 33 MB) and the second's (about 67 MB)
+    # do not fit the budget together
+    ctx = eg.Context(0, hbm_budget=80 << 20)
+    ctx.rmat(14, 1 << 20, 5).build(eg.CSR | eg.CSC).free()
+    g = ctx.rmat(15, 2 << 20, 5).build(eg.CSR | eg.CSC)
+    assert g.adj(eg.CSR)[0][-1] == 2 << 20
+    ctx.close()
