@@ -1073,7 +1073,9 @@ struct MsCounters {
     unsigned long long tdeg;  // sum over new (vertex, source) pairs of the vertex's out-degree
     unsigned long long disc;  // new (vertex, source) pairs
     uint32_t count;           // vertices with a nonzero new word
-    uint32_t nbig;            // frontier vertices deferred to k_ms_push_big
+    uint32_t nbig;            // frontier vertices deferred to k_ms_push_big; pull: k_msp_mid's list
+    uint32_t nhuge;           // pull: k_msp_heavy's list
+    uint32_t qlen;            // ids listed by k_ms_queue
 };
 
 __global__ void k_ms_init(uint32_t n, unsigned long long *seen, unsigned long long *front) {
@@ -1103,8 +1105,7 @@ struct MsGState {
 // Roots: seen/front bits, level 1, and the first frontier (distinct roots)
 // with its statistics.  One block of 64 threads.
 __global__ void k_ms_roots(const uint32_t *roots, int k, uint32_t n, unsigned long long *seen, unsigned long long *front,
-                           int32_t *levels, const uint32_t *__restrict__ deg, uint32_t *queue, MsGState *st,
-                           unsigned long long m) {
+                           int32_t *levels, const uint32_t *__restrict__ deg, MsGState *st, unsigned long long m) {
     __shared__ unsigned int s_count;
     __shared__ unsigned long long s_fdeg, s_rdeg;
     const int s = threadIdx.x;
@@ -1121,8 +1122,8 @@ __global__ void k_ms_roots(const uint32_t *roots, int k, uint32_t n, unsigned lo
         if (levels) levels[(uint64_t)s * n + r] = 1;
         const unsigned long long d = deg[r];
         atomicAdd(&s_rdeg, d);
-        if (!was) {  // the first source at this vertex lists it
-            queue[atomicAdd(&s_count, 1u)] = r;
+        if (!was) {  // the first source at this vertex counts it
+            atomicAdd(&s_count, 1u);
             atomicAdd(&s_fdeg, d);
         }
     }
@@ -1149,6 +1150,48 @@ __global__ void k_msg_prep(MsGState *st, MsCounters *cnt) {
     cnt->disc = 0;
     cnt->count = 0;
     cnt->nbig = 0;
+    cnt->nhuge = 0;
+    cnt->qlen = 0;
+}
+
+// Push levels: lists the vertices with a nonzero frontier word (four per
+// thread, one atomic per 1024 vertices).  The fold used to append them on
+// every level, one atomic per warp on the one counter.
+__global__ void __launch_bounds__(256) k_ms_queue(uint32_t n, const unsigned long long *__restrict__ front,
+                                                  uint32_t *queue, const MsGState *st, MsCounters *cnt) {
+    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_base;
+    if (st->pull) return;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t b0 = blockIdx.x * 1024ull; b0 < n; b0 += gridDim.x * 1024ull) {
+        const uint64_t v0 = b0 + warp * 128u + lane;
+        uint32_t ball[4], c = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint64_t v = v0 + 32u * i;
+            ball[i] = __ballot_sync(EG_FULL_MASK, v < n && front[v] != 0ull);
+            c += __popc(ball[i]);
+        }
+        if (lane == 0) s_warp[warp] = c;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t t = 0;
+            for (int w = 0; w < 8; w++) {
+                const uint32_t x = s_warp[w];
+                s_warp[w] = t;
+                t += x;
+            }
+            s_base = t ? atomicAdd(&cnt->qlen, t) : 0u;
+        }
+        __syncthreads();
+        uint32_t pos = s_base + s_warp[warp];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if ((ball[i] >> lane) & 1u) queue[pos + __popc(ball[i] & eg_lanemask_lt())] = (uint32_t)(v0 + 32u * i);
+            pos += __popc(ball[i]);
+        }
+        __syncthreads();  // s_warp and s_base are rewritten for the next 1024
+    }
 }
 
 // Pull: a vertex ORs the frontier words of its in-neighbours, stopping early
@@ -1230,54 +1273,77 @@ __global__ void k_msg_end(MsGState *st, const MsCounters *cnt, cudaGraphConditio
 }
 
 // Folds the new words into seen, records levels, makes them the frontier and
-// lists the frontier vertices for a following push step.
-__global__ void k_ms_fold(uint32_t n, int k, unsigned long long *seen, unsigned long long *front,
-                          unsigned long long *next, int clear_next, int32_t *levels, const MsGState *st,
-                          const uint32_t *__restrict__ deg, uint32_t *queue, MsCounters *cnt) {
+// counts it.  The warp writes the levels source by source (a row of levels is
+// one source's), so that a store covers up to 32 consecutive words; every
+// lane walking its own word's sources wrote 32 rows at once, and four
+// atomics per warp met on the counters (64 sources, undirected RMAT-20:
+// 694 us in 7 levels, now 220).
+__global__ void __launch_bounds__(256) k_ms_fold(uint32_t n, unsigned long long *seen, unsigned long long *front,
+                                                 unsigned long long *next, int32_t *levels, const MsGState *st,
+                                                 const uint32_t *__restrict__ deg, MsCounters *cnt) {
     const int32_t lvl = st->lvl + 1;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lt = eg_lanemask_lt();
-    uint32_t stride = gridDim.x * blockDim.x;
-    // uniform trip count per warp for the ballots
-    for (uint32_t v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); v0 < n; v0 += stride) {
-        const uint32_t v = v0 + lane;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    unsigned long long sum[3] = {0ull, 0ull, 0ull};  // out-degrees, out-degrees per new pair, new pairs
+    uint32_t count = 0;
+    // uniform trip count per warp for the collectives
+    for (uint64_t v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); v0 < n; v0 += stride) {
+        const uint64_t v = v0 + lane;
         unsigned long long x = 0ull;
         if (v < n) {
-            x = next[v] & ~seen[v];
-            if (clear_next) next[v] = 0ull;
-            front[v] = x;
+            x = next[v];
             if (x) {
-                seen[v] |= x;
-                if (levels) {
-                    unsigned long long y = x;
-                    while (y) {
-                        int s = __ffsll((long long)y) - 1;
-                        y &= y - 1;
-                        levels[(uint64_t)s * n + v] = lvl;
-                    }
+                next[v] = 0ull;
+                const unsigned long long s = seen[v];
+                x &= ~s;
+                if (x) seen[v] = s | x;
+            }
+            front[v] = x;
+        }
+        if (!__any_sync(EG_FULL_MASK, x != 0ull)) continue;
+        if (x) {
+            const unsigned long long d = deg[v], pc = (unsigned long long)__popcll((long long)x);
+            sum[0] += d;
+            sum[1] += d * pc;
+            sum[2] += pc;
+            count++;
+        }
+        if (levels) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t mine = (uint32_t)(x >> (32 * h));
+                uint32_t any = __reduce_or_sync(EG_FULL_MASK, mine);
+                while (any) {
+                    const uint32_t s = (uint32_t)__ffs(any) - 1;
+                    any &= any - 1;
+                    if ((mine >> s) & 1u) levels[(uint64_t)(32 * h + s) * n + v] = lvl;
                 }
             }
         }
-        const uint32_t ball = __ballot_sync(EG_FULL_MASK, x != 0ull);
-        if (ball) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&cnt->count, __popc(ball));
-            base = __shfl_sync(EG_FULL_MASK, base, 0);
-            unsigned long long d = x ? (unsigned long long)deg[v] : 0ull;
-            unsigned long long pc = (unsigned long long)__popcll((long long)x);
-            unsigned long long td = d * pc;
-            if (x) queue[base + __popc(ball & lt)] = v;
+    }
+    __shared__ unsigned long long s_sum[8][3];
+    __shared__ uint32_t s_cnt[8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                d += __shfl_down_sync(EG_FULL_MASK, d, o);
-                td += __shfl_down_sync(EG_FULL_MASK, td, o);
-                pc += __shfl_down_sync(EG_FULL_MASK, pc, o);
-            }
-            if (lane == 0) {
-                atomicAdd(&cnt->deg, d);
-                atomicAdd(&cnt->tdeg, td);
-                atomicAdd(&cnt->disc, pc);
-            }
+    for (int o = 16; o > 0; o >>= 1) {
+        count += __shfl_down_sync(EG_FULL_MASK, count, o);
+#pragma unroll
+        for (int i = 0; i < 3; i++) sum[i] += __shfl_down_sync(EG_FULL_MASK, sum[i], o);
+    }
+    if (lane == 0) {
+        s_cnt[warp] = count;
+        for (int i = 0; i < 3; i++) s_sum[warp][i] = sum[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) {
+            count += s_cnt[w];
+            for (int i = 0; i < 3; i++) sum[i] += s_sum[w][i];
+        }
+        if (count) {
+            atomicAdd(&cnt->count, count);
+            atomicAdd(&cnt->deg, sum[0]);
+            atomicAdd(&cnt->tdeg, sum[1]);
+            atomicAdd(&cnt->disc, sum[2]);
         }
     }
 }
@@ -1287,7 +1353,7 @@ __global__ void k_ms_fold(uint32_t n, int k, unsigned long long *seen, unsigned 
 // is prep (direction), push (+ hubs in chunks) or the two-part pull, fold,
 // and end (counters into the state, loop condition).  Valid while the
 // buffers and k it was captured with (key) stay the same.
-static int msbfs_graph_build(eg_graph *g, const void *const key[8], const eg_adj *in_adj, int k,
+static int msbfs_graph_build(eg_graph *g, const void *const key[8], const eg_adj *in_adj,
                              unsigned long long all, unsigned long long *seen, unsigned long long *front,
                              unsigned long long *next, uint32_t *queue, uint32_t *big, uint32_t *bigoff, int32_t *levels,
                              MsGState *st, MsCounters *cnt) {
@@ -1315,17 +1381,20 @@ static int msbfs_graph_build(eg_graph *g, const void *const key[8], const eg_adj
     const uint32_t blocks = (uint32_t)ctx->sm_count * 8;
     EG_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     k_msg_prep<<<1, 1, 0, ctx->stream>>>(st, cnt);
+    k_ms_queue<<<blocks, 256, 0, ctx->stream>>>(n, front, queue, st, cnt);
     k_ms_push<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(g->csr.ptr), bp<uint32_t>(g->csr.col), queue, st, seen,
                                                front, next, big, cnt);
     k_big_offsets<<<1, 1024, 0, ctx->stream>>>(big, &cnt->nbig, 1u, bp<uint32_t>(g->csr.ptr), EG_BFS_CHUNK, bigoff);
     k_ms_push_big<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(g->csr.ptr), bp<uint32_t>(g->csr.col), big, bigoff,
                                                    seen, front, next, cnt);
-    // the heavy list reuses the push side list (idle in a pull level)
+    // the pull's lists reuse the push side list and queue (idle in a pull level)
     k_msp_light<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), n, all, seen,
                                                  front, next, big, &cnt->nbig, &st->pull);
+    k_msp_mid<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), all, seen, front,
+                                               next, big, &cnt->nbig, queue, &cnt->nhuge, &st->pull);
     k_msp_heavy<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), all, seen, front,
-                                                 next, big, &cnt->nbig, &st->pull);
-    k_ms_fold<<<blocks, 256, 0, ctx->stream>>>(n, k, seen, front, next, 1, levels, st, deg, queue, cnt);
+                                                 next, queue, &cnt->nhuge, &st->pull);
+    k_ms_fold<<<blocks, 256, 0, ctx->stream>>>(n, seen, front, next, levels, st, deg, cnt);
     k_msg_end<<<1, 1, 0, ctx->stream>>>(st, cnt, handle);
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &body);
     if (ce != cudaSuccess) return eg_fail(EG_ECUDA, "multi-source BFS capture: %s", cudaGetErrorString(ce));
@@ -1374,14 +1443,14 @@ extern "C" int eg_bfs_multi(eg_graph *g, const uint32_t *roots, int k, int32_t *
     bool same = g->msg.exec != nullptr;
     for (int i = 0; i < 8 && same; i++) same = g->msg.key[i] == key[i];
     if (!same)
-        EG_TRY(msbfs_graph_build(g, key, in_adj, k, all, seen, front, next, queue, big, bigoff, levels, st, cnt));
+        EG_TRY(msbfs_graph_build(g, key, in_adj, all, seen, front, next, queue, big, bigoff, levels, st, cnt));
     EG_CUDA(cudaMemcpyAsync(d_roots, roots, (uint64_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
     EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     if (levels) EG_CUDA(cudaMemsetAsync(levels, 0, (uint64_t)k * n * 4, ctx->stream));
     k_ms_init<<<blocks_for(ctx, n), 256, 0, ctx->stream>>>(n, seen, front);
     EG_LAUNCHED(ctx);
     EG_CUDA(cudaMemsetAsync(next, 0, (uint64_t)n * 8, ctx->stream));
-    k_ms_roots<<<1, 64, 0, ctx->stream>>>(d_roots, k, n, seen, front, levels, deg, queue, st, g->m);
+    k_ms_roots<<<1, 64, 0, ctx->stream>>>(d_roots, k, n, seen, front, levels, deg, st, g->m);
     EG_LAUNCHED(ctx);
     EG_CUDA(cudaGraphLaunch(g->msg.exec, ctx->stream));
     ctx->launches++;

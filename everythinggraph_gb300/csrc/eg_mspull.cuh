@@ -7,17 +7,24 @@
 //
 // A serial scan per vertex is fine for the common low-degree vertex but not
 // for a hub whose sources stay unsatisfied (it would read its whole in-list,
-// 10^5..10^6 entries, from one thread).  So the level runs in two parts:
-//   k_msp_light  one thread per vertex scans at most EG_MSP_LIGHT in-entries;
-//                a vertex still unsatisfied with entries left goes to the
-//                heavy list, its partial word parked in next[v];
-//   k_msp_heavy  one CTA per heavy vertex scans the rest 1024 entries per
-//                step (4 per thread, coalesced), ORs the warps' words in
-//                shared memory and stops once the need is met.
+// 10^5..10^6 entries, from one thread).  So the level runs in three parts:
+//   k_msp_light  one thread per vertex scans at most EG_MSP_LIGHT in-entries,
+//                four per step with all their loads in flight; a vertex still
+//                unsatisfied with entries left goes to the heavy list, its
+//                partial word parked in next[v];
+//   k_msp_mid    one warp per heavy vertex scans up to EG_MSP_MID more, 128
+//                per step (a CTA per vertex spent its barriers and idle
+//                threads on lists of 33 to 1000 entries, most of the heavy
+//                list: 488 us per 64-source batch on undirected RMAT-20, now
+//                117 and 169 for the rest);
+//   k_msp_heavy  one CTA per vertex still unsatisfied scans the rest 1024
+//                entries per step (4 per thread, coalesced), ORs the warps'
+//                words in shared memory and stops once the need is met.
 #pragma once
 #include "eg_internal.cuh"
 
 #define EG_MSP_LIGHT 32u
+#define EG_MSP_MID 1024u
 
 namespace {
 
@@ -40,10 +47,14 @@ __global__ void __launch_bounds__(256) k_msp_light(const uint32_t *__restrict__ 
             if (need) {
                 const uint32_t b = ptr[v], e = ptr[v + 1];
                 const uint32_t lim = e - b > EG_MSP_LIGHT ? b + EG_MSP_LIGHT : e;
-                for (uint32_t p = b; p < lim; p++) {
-                    acc |= __ldg(front + col[p]);
+                uint32_t p = b;
+                for (; p + 4 <= lim; p += 4) {
+                    const uint32_t u0 = col[p], u1 = col[p + 1], u2 = col[p + 2], u3 = col[p + 3];
+                    acc |= (__ldg(front + u0) | __ldg(front + u1)) | (__ldg(front + u2) | __ldg(front + u3));
                     if ((acc & need) == need) break;
                 }
+                if ((acc & need) != need)
+                    for (; p < lim; p++) acc |= __ldg(front + col[p]);
                 hv = (acc & need) != need && lim < e;
             }
             next[v] = hv ? acc : (acc & need);
@@ -58,23 +69,61 @@ __global__ void __launch_bounds__(256) k_msp_light(const uint32_t *__restrict__ 
     }
 }
 
+// huge (room for n ids) lists the vertices left to k_msp_heavy.
+__global__ void __launch_bounds__(256) k_msp_mid(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
+                                                 unsigned long long all, const unsigned long long *__restrict__ seen,
+                                                 const unsigned long long *__restrict__ front,
+                                                 unsigned long long *__restrict__ next,
+                                                 const uint32_t *__restrict__ heavy, const uint32_t *heavy_count,
+                                                 uint32_t *__restrict__ huge, uint32_t *huge_count,
+                                                 const int *gate = nullptr) {
+    if (gate && !*gate) return;
+    const uint32_t nh = *(volatile const uint32_t *)heavy_count;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nh; i += warps) {
+        const uint32_t v = heavy[i];
+        const unsigned long long need = all & ~seen[v];
+        unsigned long long tot = next[v];  // the light scan's partial word
+        const uint32_t b = ptr[v] + EG_MSP_LIGHT, e = ptr[v + 1];
+        const uint32_t lim = e - b > EG_MSP_MID ? b + EG_MSP_MID : e;
+        for (uint32_t base = b; base < lim; base += 128u) {
+            unsigned long long acc = 0ull;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t p = base + k * 32u + lane;
+                if (p < lim) acc |= __ldg(front + col[p]);
+            }
+            const uint32_t lo = __reduce_or_sync(EG_FULL_MASK, (uint32_t)acc);
+            const uint32_t hi = __reduce_or_sync(EG_FULL_MASK, (uint32_t)(acc >> 32));
+            tot |= ((unsigned long long)hi << 32) | lo;
+            if ((tot & need) == need) break;
+        }
+        const bool more = (tot & need) != need && lim < e;
+        if (lane == 0) {
+            next[v] = more ? tot : (tot & need);
+            if (more) huge[atomicAdd(huge_count, 1u)] = v;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256) k_msp_heavy(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
                                                    unsigned long long all, const unsigned long long *__restrict__ seen,
                                                    const unsigned long long *__restrict__ front,
                                                    unsigned long long *__restrict__ next,
-                                                   const uint32_t *__restrict__ heavy, const uint32_t *heavy_count,
+                                                   const uint32_t *__restrict__ huge, const uint32_t *huge_count,
                                                    const int *gate = nullptr) {
     __shared__ unsigned long long s_acc;
     if (gate && !*gate) return;
-    const uint32_t nh = *(volatile const uint32_t *)heavy_count;
+    const uint32_t nh = *(volatile const uint32_t *)huge_count;
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t i = blockIdx.x; i < nh; i += gridDim.x) {
-        const uint32_t v = heavy[i];
+        const uint32_t v = huge[i];
         const unsigned long long need = all & ~seen[v];
-        if (threadIdx.x == 0) s_acc = next[v];  // the light scan's partial word
+        if (threadIdx.x == 0) s_acc = next[v];  // the earlier scans' partial word
         __syncthreads();
         const uint32_t e = ptr[v + 1];
-        for (uint32_t base = ptr[v] + EG_MSP_LIGHT; base < e; base += 1024u) {
+        for (uint32_t base = ptr[v] + EG_MSP_LIGHT + EG_MSP_MID; base < e; base += 1024u) {
             unsigned long long acc = 0ull;
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) {

@@ -48,7 +48,7 @@ struct SvCounters {
     uint32_t qsize;
     uint32_t nbig;
     uint32_t grab, grab_big;  // SSSP work units handed out this step
-    uint32_t pad;
+    uint32_t nhuge;           // BFS pull: k_msp_heavy's list
 };
 
 // ------------------------------------------------------------------ BFS engine
@@ -777,8 +777,12 @@ static int sv_bfs_advance(eg_server *s, bool *progress, bool launch, bool *launc
         k_msp_light<<<sv_blocks(ctx, n), 256, 0, st>>>(bp<uint32_t>(g->csc.ptr), bp<uint32_t>(g->csc.col), n, live, seen,
                                                        front, next, bbig, &bcnt->nbig);
         EG_LAUNCHED(ctx);
+        // the lists: the push side list and the queue, idle in a pull level
+        k_msp_mid<<<(uint32_t)ctx->sm_count * 8, 256, 0, st>>>(bp<uint32_t>(g->csc.ptr), bp<uint32_t>(g->csc.col), live,
+                                                               seen, front, next, bbig, &bcnt->nbig, bq, &bcnt->nhuge);
+        EG_LAUNCHED(ctx);
         k_msp_heavy<<<(uint32_t)ctx->sm_count * 8, 256, 0, st>>>(bp<uint32_t>(g->csc.ptr), bp<uint32_t>(g->csc.col), live,
-                                                                 seen, front, next, bbig, &bcnt->nbig);
+                                                                 seen, front, next, bq, &bcnt->nhuge);
         EG_LAUNCHED(ctx);
     } else {
         k_sv_front_queue<<<sv_blocks(ctx, n), 256, 0, st>>>(front, n, bq, bcnt);
