@@ -217,6 +217,11 @@ struct eg_graph {
     eg_buf msbfs_work;
     eg_buf sssp_work;
     eg_buf ppr_work;
+    // batched personalised PageRank's work list over the CSC (eg_ppr_plan):
+    // parts of the long rows, the long rows, the other rows longest first
+    eg_buf ppr_long, ppr_multi, ppr_order;
+    uint32_t ppr_nlong = 0, ppr_nmulti = 0, ppr_nrows = 0;
+    bool ppr_planned = false;
     eg_bfs_graph bfsg[2 * EG_OUT_SLOTS];  // [slot * 2 + with parents]
     eg_bfs_graph prg;      // PageRank iterations (key: options and buffers)
     eg_bfs_graph msg;      // multi-source BFS level loop
@@ -246,6 +251,8 @@ int eg_radix_sort(eg_ctx *ctx, uint32_t *k_in, uint32_t *v_in, uint32_t *k_tmp, 
                   int bits, uint32_t **k_out, uint32_t **v_out);
 // builds g->csc_p / perm / deg_p from the CSC and out-degrees (once)
 int eg_build_relabeled_csc(eg_graph *g);
+// builds the batched personalised PageRank's work list (once per CSC)
+int eg_ppr_plan(eg_graph *g);
 // builds g->pcol with partitions of 2^shift rows from g->csc_p (once per shift)
 int eg_build_pcols(eg_graph *g, uint32_t shift);
 

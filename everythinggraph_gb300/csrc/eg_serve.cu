@@ -515,11 +515,11 @@ extern "C" int eg_serve_open(eg_graph *g, const eg_serve_opts *opts, eg_server *
     if (rc == EG_OK)
         rc = eg_buf_ensure(ctx, s->sssp_buf, (uint64_t)n * 4 * SV_SSSP_SLOTS + (uint64_t)n * 8 * 2 + (uint64_t)((n + 31) / 32) * 4 * 2 +
                                                  (uint64_t)n * 4 * 4 + 4);
-    // PPR: R, X, Y [n][32] | parts
-    const uint64_t ptiles = g->m ? (g->m + EG_PPR_TILE - 1) / EG_PPR_TILE : 0;
+    // PPR: R, X, Y [n][32] | part sums | block partials
+    if (rc == EG_OK) rc = eg_ppr_plan(g);
     if (rc == EG_OK)
-        rc = eg_buf_ensure(ctx, s->ppr_buf, (uint64_t)n * 4 * EG_PPR_LANES * 3 + ptiles * EG_PPR_LANES * 4 * 2 +
-                                                 ((ptiles + 63) & ~63ull) * 4 + (uint64_t)ctx->sm_count * 4 * 32 * 16 + 256);
+        rc = eg_buf_ensure(ctx, s->ppr_buf, (uint64_t)n * 4 * EG_PPR_LANES * 3 + (uint64_t)g->ppr_nlong * EG_PPR_LANES * 4 +
+                                                 (uint64_t)ctx->sm_count * 4 * 32 * 16 + 256);
     if (rc == EG_OK) rc = eg_buf_ensure(ctx, s->small, 64 * 1024);
     if (rc == EG_OK) rc = eg_buf_ensure(ctx, s->wts_buf, g->m * 4 + 16);
     if (rc == EG_OK) rc = eg_fill_weights(g, eg_make_wrule(&o.weights), bp<uint32_t>(s->wts_buf));
@@ -1046,18 +1046,19 @@ static int sv_ppr_advance(eg_server *s, bool *progress, bool launch, bool *launc
         *progress = true;
     }
     if (!s->ppr_mask) return EG_OK;
-    const uint32_t pm = (uint32_t)g->m;
-    const uint32_t ptiles = pm ? eg_div_up(pm, EG_PPR_TILE) : 0;
-    float *phv = Y + (uint64_t)n * EG_PPR_LANES, *ptv = phv + (uint64_t)ptiles * EG_PPR_LANES;
-    uint32_t *phr = reinterpret_cast<uint32_t *>(ptv + (uint64_t)ptiles * EG_PPR_LANES);
-    double2 *ppart = reinterpret_cast<double2 *>(phr + ((ptiles + 63) & ~63u));
+    float *psum = Y + (uint64_t)n * EG_PPR_LANES;
+    double2 *ppart = reinterpret_cast<double2 *>(psum + (uint64_t)g->ppr_nlong * EG_PPR_LANES);
     const uint32_t fb = (uint32_t)ctx->sm_count * 4;
-    const uint32_t rb = ptiles ? eg_div_up((uint64_t)ptiles * 32, 256) : 0;
     EG_CUDA(cudaEventRecord(s->ev_begin[E_PPR], st));
-    if (rb) {
-        k_ppr_rows<<<rb, 256, 0, st>>>(bp<uint32_t>(g->csc.rid), bp<uint32_t>(g->csc.col), pm, ptiles, X, Y, phv, ptv, phr);
+    if (g->ppr_nlong + g->ppr_nrows) {
+        k_ppr_rows<<<(uint32_t)ctx->sm_count * EG_PPR_MINB, 256, 0, st>>>(
+            bp<uint32_t>(g->csc.ptr), bp<uint32_t>(g->csc.col), bp<uint4>(g->ppr_long), g->ppr_nlong,
+            bp<uint32_t>(g->ppr_order), g->ppr_nrows, X, Y, psum);
         EG_LAUNCHED(ctx);
-        k_ppr_fixup<<<rb, 256, 0, st>>>(bp<uint32_t>(g->csc.ptr), ptiles, phr, phv, ptv, Y);
+    }
+    if (g->ppr_nmulti) {
+        k_ppr_fixup<<<eg_div_up((uint64_t)g->ppr_nmulti * 32, 256), 256, 0, st>>>(bp<uint4>(g->ppr_multi), g->ppr_nmulti,
+                                                                                  psum, Y);
         EG_LAUNCHED(ctx);
     }
     k_ppr_empty<<<(uint32_t)ctx->sm_count * 8, 256, 0, st>>>(bp<uint32_t>(g->csc.ptr), n, Y);
@@ -1066,7 +1067,7 @@ static int sv_ppr_advance(eg_server *s, bool *progress, bool launch, bool *launc
     EG_LAUNCHED(ctx);
     k_ppr_finish<<<fb, 256, 0, st>>>(Y, deg, n, s->opts.ppr_damping, d_ppr, R, X, ppart);
     EG_LAUNCHED(ctx);
-    k_ppr_reduce<<<1, 32, 0, st>>>(ppart, fb, d_ppr, 1);
+    k_ppr_reduce<<<EG_PPR_LANES, 128, 0, st>>>(ppart, fb, d_ppr, 1);
     EG_LAUNCHED(ctx);
     EG_CUDA(cudaMemcpyAsync(hp, d_ppr, sizeof(PprQ) * EG_PPR_LANES, cudaMemcpyDeviceToHost, st));
     EG_CUDA(cudaEventRecord(s->ev_end[E_PPR], st));
