@@ -216,7 +216,6 @@ extern "C" int eg_graph_load_layouts(eg_graph *g, const char *path, int *hit) {
     // derived copies follow the layouts they were made from
     g->first_in_src = nullptr;
     g->ppr_planned = false;
-    g->wcc_list_src = nullptr;
     g->relabeled = false;
     g->sb.blocks = g->sb.shift = 0;
     g->sbp.blocks = g->sbp.shift = 0;

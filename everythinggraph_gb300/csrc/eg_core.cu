@@ -476,8 +476,7 @@ extern "C" void eg_graph_free(eg_graph *g) {
                       &g->grid_order,   &g->grid_units,  &g->grid_off,    &g->grid_vals,   &g->grid_acc,
                       &g->esrc,         &g->edst,        &g->edge_work,
                       &g->pcol.dst,     &g->pcol.ridx,  &g->pcol.crun,   &g->pcol.rsrc,   &g->pcol.seg,
-                      &g->pcol.acc,     &g->pcol.ticket,  &g->wcc_list,
-                      &g->ppr_long,     &g->ppr_multi,   &g->ppr_order};
+                      &g->pcol.acc,     &g->pcol.ticket,  &g->ppr_long,     &g->ppr_multi,   &g->ppr_order};
     for (eg_buf *b : bufs) eg_buf_free(c, *b);
     for (eg_bfs_graph &bg : g->bfsg) {
         if (bg.exec) cudaGraphExecDestroy(bg.exec);
@@ -1100,7 +1099,6 @@ static int build_adj_pair(eg_graph *g, bool want_csc) {
     BTRY(rows_from_rid(ctx, bp<uint32_t>(g->csr.rid), M, n, bp<uint32_t>(g->out_deg), bp<uint32_t>(g->csr.ptr)));
     g->built |= EG_LAYOUT_CSR;
     g->first_in_src = nullptr;
-    g->wcc_list_src = nullptr;
     if (want_csc) {
         // CSC: stable sort of the CSR entries by dst, value src
         if (M) {
@@ -1112,8 +1110,7 @@ static int build_adj_pair(eg_graph *g, bool want_csc) {
         BTRY(rows_from_rid(ctx, bp<uint32_t>(g->csc.rid), M, n, bp<uint32_t>(g->in_deg), bp<uint32_t>(g->csc.ptr)));
         g->built |= EG_LAYOUT_CSC;
         g->first_in_src = nullptr;
-        g->wcc_list_src = nullptr;
-        g->relabeled = false;  // so do PageRank's relabelled copy
+            g->relabeled = false;  // so do PageRank's relabelled copy
         g->ppr_planned = false;
         g->sb.blocks = 0;  // the source-blocked copies follow the CSC
         g->sb.shift = 0;
