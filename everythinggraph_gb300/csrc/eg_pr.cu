@@ -19,6 +19,7 @@
 //   k_coo_empty_range, k_coo_fixup  rows without entries, rows split between tiles
 //   k_pr_residual          (with a tolerance) the L1 change, coalesced
 //   k_pr_reduce            FP64 residual / dangling mass -> next base, stop flag
+// On small graphs all iterations are one cooperative launch (eg_prsmall.cuh).
 // contrib[u] = prev[u] / (float)deg[u] is the reference's per-edge quotient
 // (pagerank_simple.c:78), computed once per vertex instead of once per edge.
 // Algorithmic bytes per iteration: 8 per entry (row id + column) and 16 per
@@ -57,6 +58,8 @@ struct eg_pr_dev {
     double residual;
     double dangling;
 };
+
+#include "eg_prsmall.cuh"
 
 // Teleport set of a single personalised PageRank query: up to
 // EG_PPR1_SEEDS distinct vertices (relabelled ids) with their multiplicity.
@@ -602,6 +605,56 @@ static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st
 // Shared by eg_pagerank and eg_ppr: the iterations over the relabelled CSC,
 // then the ranks back in the original vertex order.  `ps` (in relabelled
 // ids) selects the personalised teleport; its total multiplicity divides it.
+// Whether a run goes to k_pr_small: plain PageRank on the default schedule, of
+// a size where its one launch is faster than the launches per iteration (the
+// figures are beside the kernel).
+static bool pr_small(const eg_graph *g, const eg_pr_opts &o) {
+    if (!g->m || o.compensated || g->row_cfg != 0 || g->pr_kernel != 0 || pr_block_log2(g, o)) return false;
+    return g->n <= EG_PRS_STAGE_N ? g->m <= EG_PRS_STAGE_M : g->n <= EG_PRS_MAX_N && g->m <= EG_PRS_MAX_M;
+}
+
+static int pr_run_small(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr_stats *stats) {
+    eg_ctx *ctx = g->ctx;
+    const uint32_t n = g->n, m = (uint32_t)g->m;
+    const uint32_t want = eg_div_up(m, EG_PRS_SHARE), G = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
+    for (eg_buf *b : {&g->rank, &g->rank_p, &g->contrib0, &g->contrib1}) EG_TRY(eg_buf_ensure(ctx, *b, (uint64_t)n * 4));
+    EG_TRY(eg_buf_ensure(ctx, g->pr_part, 2ull * G * sizeof(float4)));
+    eg_pr_dev *st = bp<eg_pr_dev>(g->pr_stats);
+    const bool reduce = o.tolerance > 0.0 || o.dangling;
+    const bool stage = n <= EG_PRS_STAGE_N;
+    const uint64_t cw = stage ? 2 : 4;  // bytes of a kept column
+    const uint64_t fixed = stage ? (n * 4ull + 15) & ~15ull : 0, cap = (220 * 1024 - fixed) / cw;
+    const uint64_t share = (m + (uint64_t)EG_PRS_ROW * g->csc_p_rows) / G + EG_PRS_WARP;  // a longer last row's rest stays in memory
+    PrSmall a{bp<uint32_t>(g->csc_p.ptr), bp<uint32_t>(g->csc_p.col), bp<uint32_t>(g->deg_p), bp<uint32_t>(g->perm),
+              n, g->csc_p_rows, m, o.deg_multiplier, o.iterations, o.swap, o.dangling, o.damping,
+              o.prev_init < 0.f ? 1.0f / (float)n : o.prev_init, (1.0 - (double)o.damping) / (double)n,
+              (double)o.damping / (double)n, o.tolerance, bp<float>(g->contrib0), bp<float>(g->contrib1),
+              bp<float>(g->rank_p), bp<float>(g->rank), bp<float4>(g->pr_part), st,
+              (uint32_t)(share < cap ? share : cap)};
+    const size_t smem = (size_t)(fixed + ((a.cap * cw + 15) & ~15ull));
+    const void *fn = stage ? (reduce ? (const void *)k_pr_small<true, true> : (const void *)k_pr_small<false, true>)
+                           : (reduce ? (const void *)k_pr_small<true, false> : (const void *)k_pr_small<false, false>);
+    EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void *args[] = {&a};
+    EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
+    EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(EG_PRS_THREADS), args, smem, ctx->stream));
+    ctx->launches++;
+    EG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
+    eg_pr_dev *h = reinterpret_cast<eg_pr_dev *>(ctx->h_pinned);
+    EG_TRY(eg_readback(ctx, h, st, sizeof(eg_pr_dev), ctx->stream));
+    if (rank_out) EG_CUDA(cudaMemcpyAsync(rank_out, g->rank.p, (uint64_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    EG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (stats) {
+        stats->iterations_run = h->iters;
+        stats->residual = o.tolerance > 0.0 ? h->residual : 0.0;
+        stats->dangling_mass = reduce ? h->dangling : 0.0;
+        EG_CUDA(cudaEventElapsedTime(&stats->ms, ctx->ev0, ctx->ev1));
+        // the launch holds the row sums of every iteration
+        stats->row_kernel_ms = o.use_graph || !h->iters ? 0.f : stats->ms / (float)h->iters;
+    }
+    return EG_OK;
+}
+
 static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t seed_total, float *rank_out,
                   eg_pr_stats *stats) {
     eg_ctx *ctx = g->ctx;
@@ -719,6 +772,7 @@ extern "C" int eg_pagerank(eg_graph *g, const eg_pr_opts *opts, float *rank_out,
         }
     }
     EG_TRY(pr_prepare(g, &o));
+    if (pr_small(g, o)) return pr_run_small(g, o, rank_out, stats);
     PprSeeds none;
     memset(&none, 0, sizeof(none));
     return pr_run(g, o, none, 0, rank_out, stats);

@@ -177,7 +177,9 @@ typedef struct {
     double dangling_mass; /* FP64 mass on out-degree-0 vertices, last iterate */
     float ms;             /* device time of the iterations */
     float row_kernel_ms;  /* mean device time of one row-sum kernel launch (up to
-                             the first 8 iterations; 0 when use_graph) */
+                             the first 8 iterations; 0 when use_graph; small
+                             graphs run all iterations in one launch: its time
+                             per iteration) */
 } eg_pr_stats;
 void eg_pr_opts_default(eg_pr_opts *o);
 int eg_pagerank(eg_graph *g, const eg_pr_opts *opts, float *rank_out, eg_pr_stats *stats);
