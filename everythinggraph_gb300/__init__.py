@@ -328,8 +328,7 @@ class Graph:
 
     def bfs(self, root, direction="auto", switch_divisor=None, parents=False, copy_out=True, host_loop=None,
             level_out=None, parent_out=None):
-        """host_loop: None = the form eg_graph_tune kept (else the CUDA graph),
-        False = CUDA-graph level loop, True = host-driven level loop.
+        """host_loop: accepted, without effect (one level loop serves both forms).
         switch_divisor: None = the divisor eg_graph_tune kept (else 40, the
         reference's).
         level_out / parent_out: int32 arrays of n elements to fill (e.g. from

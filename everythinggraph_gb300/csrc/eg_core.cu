@@ -478,10 +478,6 @@ extern "C" void eg_graph_free(eg_graph *g) {
                       &g->pcol.dst,     &g->pcol.ridx,  &g->pcol.crun,   &g->pcol.rsrc,   &g->pcol.seg,
                       &g->pcol.acc,     &g->pcol.ticket,  &g->ppr_long,     &g->ppr_multi,   &g->ppr_order};
     for (eg_buf *b : bufs) eg_buf_free(c, *b);
-    for (eg_bfs_graph &bg : g->bfsg) {
-        if (bg.exec) cudaGraphExecDestroy(bg.exec);
-        if (bg.graph) cudaGraphDestroy(bg.graph);
-    }
     for (eg_bfs_graph *bg : {&g->prg, &g->msg, &g->ssg, &g->s1g, &g->ppg}) {
         if (bg->exec) cudaGraphExecDestroy(bg->exec);
         if (bg->graph) cudaGraphDestroy(bg->graph);

@@ -6,10 +6,7 @@
 //                shuffle search, so every lane has an edge whatever the
 //                degrees (one warp per vertex leaves most lanes idle on
 //                low-degree frontiers).
-// k_bm_queue     frontier bitmap -> vertex-id queue: a thread per bitmap
-//                word, a block-wide exclusive scan of the words' popcounts
-//                places the ids, one atomic per block reserves the space;
-//                optionally clears the words it read.
+// eg_list_find   the entry of a list with running sums that holds a place.
 #pragma once
 #include "eg_internal.cuh"
 
@@ -46,44 +43,21 @@ __device__ __forceinline__ void eg_warp_lists(uint32_t u, uint32_t b, uint32_t d
     }
 }
 
-__global__ void __launch_bounds__(256) k_bm_queue(uint32_t *__restrict__ bm, uint32_t n, uint32_t *queue,
-                                                  uint32_t *qsize, int clear) {
-    __shared__ uint32_t s_warp[8];
-    __shared__ uint32_t s_base;
-    const uint32_t nw = (n + 31) >> 5;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t w0 = blockIdx.x * blockDim.x; w0 < nw; w0 += gridDim.x * blockDim.x) {
-        const uint32_t w = w0 + threadIdx.x;
-        const uint32_t word = w < nw ? bm[w] : 0u;
-        if (clear && word) bm[w] = 0u;
-        const uint32_t c = __popc(word);
-        uint32_t x = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(EG_FULL_MASK, x, o);
-            if (lane >= (uint32_t)o) x += y;
-        }
-        if (lane == 31) s_warp[warp] = x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t t = 0;
-            for (int i = 0; i < 8; i++) {
-                const uint32_t v = s_warp[i];
-                s_warp[i] = t;
-                t += v;
-            }
-            s_base = t ? atomicAdd(qsize, t) : 0u;
-        }
-        __syncthreads();
-        uint32_t pos = s_base + s_warp[warp] + x - c;
-        uint32_t bits = word;
-        while (bits) {
-            const int bb = __ffs(bits) - 1;
-            bits &= bits - 1;
-            queue[pos++] = (w << 5) + (uint32_t)bb;
-        }
-        __syncthreads();
+// The list entry that holds place p: the last i with off[i * stride] <= p
+// (off[0] = 0), found by a whole warp, 32 probes per step.
+__device__ __forceinline__ uint32_t eg_list_find(const uint32_t *__restrict__ off, uint32_t stride, uint32_t cnt,
+                                              uint32_t p) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t i0 = 0, len = cnt;
+    while (len > 1) {
+        const uint32_t s = (len + 31) >> 5, k = lane * s;
+        const uint32_t b =
+            __ballot_sync(EG_FULL_MASK, k < len && __ldcg(off + (uint64_t)(i0 + k) * stride) <= p);
+        const uint32_t at = (31u - (uint32_t)__clz(b)) * s;  // bit 0 is set
+        i0 += at;
+        len = len - at < s ? len - at : s;
     }
+    return i0;
 }
 
 }  // namespace

@@ -115,7 +115,7 @@ struct eg_adj {
 };
 
 
-// A BFS level loop captured as a CUDA graph with a device-side while node,
+// A round or level loop captured as a CUDA graph with a device-side while node,
 // valid while the buffers it was captured with (key) stay in place.
 struct eg_bfs_graph {
     cudaGraph_t graph = nullptr;
@@ -217,14 +217,12 @@ struct eg_graph {
     eg_buf ppr_long, ppr_multi, ppr_order;
     uint32_t ppr_nlong = 0, ppr_nmulti = 0, ppr_nrows = 0;
     bool ppr_planned = false;
-    eg_bfs_graph bfsg[2 * EG_OUT_SLOTS];  // [slot * 2 + with parents]
     eg_bfs_graph prg;      // PageRank iterations (key: options and buffers)
     eg_bfs_graph msg;      // multi-source BFS level loop
     eg_bfs_graph ssg;      // batched SSSP round loop
     eg_bfs_graph s1g;      // single-source SSSP round loop
     eg_bfs_graph ppg;      // batched personalised PageRank sweep loop
     int row_cfg = 0;       // row-kernel schedule (entries per warp tile, per lane)
-    int bfs_host_loop = 0; // BFS level-loop form eg_bfs uses by default (eg_graph_tune)
     double bfs_divisor = 40.0;  // push/pull switch divisor eg_bfs uses by default (the reference's rule; eg_graph_tune)
     // SSSP edge weights of the CSR entries for one rule, materialised on first
     // use (the reference stores them in its edge records, init_all.c:661-686)
@@ -338,8 +336,8 @@ struct eg_wrule {
     __device__ __forceinline__ uint32_t extend(uint32_t du, uint32_t u, uint32_t v) const { return add(du, weight(u, v)); }
 };
 struct eg_graph;
-// Times eg_bfs's two level-loop forms on a few sampled roots (eg_bfs.cu).
-int eg_bfs_tune(eg_graph *g, float *ms_graph, float *ms_host, int *host_loop, double *divisor);
+// Times eg_bfs on sampled roots and keeps the best switch divisor (eg_bfs.cu).
+int eg_bfs_tune(eg_graph *g, float *ms, double *divisor);
 // SpMV / PageRank over the 2-D grid layout (eg_grid.cu).
 int eg_grid_spmv(eg_graph *g, int kind, uint64_t value_seed, int unit_values, const void *d_x, void *d_y);
 int eg_grid_pagerank(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr_stats *stats);

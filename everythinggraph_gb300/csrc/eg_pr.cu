@@ -846,8 +846,10 @@ extern "C" int eg_graph_tune(eg_graph *g, eg_tune_result *out) {
         }
     }
 tuned:
-    if (g->built & EG_LAYOUT_CSR)
-        EG_TRY(eg_bfs_tune(g, &r.bfs_graph_ms, &r.bfs_host_ms, &r.bfs_host_loop, &r.bfs_switch_divisor));
+    if (g->built & EG_LAYOUT_CSR) {
+        EG_TRY(eg_bfs_tune(g, &r.bfs_graph_ms, &r.bfs_switch_divisor));
+        r.bfs_host_ms = r.bfs_graph_ms;  // one form serves both
+    }
     if (out) *out = r;
     return EG_OK;
 }

@@ -14,6 +14,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "eg_frontier.cuh"
 #include "eg_internal.cuh"
 
 namespace {
@@ -110,23 +111,6 @@ __device__ __forceinline__ unsigned long long sssp_pick(const unsigned long long
     __syncthreads();
     *last = *s_last;
     return total;
-}
-
-// The list entry that holds place p: the last i with off[i * stride] <= p
-// (off[0] = 0), found by a whole warp, 32 probes per step.
-__device__ __forceinline__ uint32_t sssp_find(const uint32_t *__restrict__ off, uint32_t stride, uint32_t cnt,
-                                              uint32_t p) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t i0 = 0, len = cnt;
-    while (len > 1) {
-        const uint32_t s = (len + 31) >> 5, k = lane * s;
-        const uint32_t b =
-            __ballot_sync(EG_FULL_MASK, k < len && __ldg(off + (uint64_t)(i0 + k) * stride) <= p);
-        const uint32_t at = (31u - (uint32_t)__clz(b)) * s;  // bit 0 is set
-        i0 += at;
-        len = len - at < s ? len - at : s;
-    }
-    return i0;
 }
 
 __global__ void k_sssp_init(uint32_t n, uint32_t nw, uint32_t *dist, uint32_t root, uint32_t *bm, SsspState *st,
@@ -384,7 +368,7 @@ __global__ void __launch_bounds__(256) k_sssp_push(const uint4 *__restrict__ que
     if (first >= E) return;
     uint32_t p = (uint32_t)first;
     const uint32_t end = E - p > per ? p + per : E;
-    uint32_t i0 = sssp_find(&queue[0].x, 4u, cnt, p);
+    uint32_t i0 = eg_list_find(&queue[0].x, 4u, cnt, p);
     for (; p < end; i0 += 32) {
         uint4 q = make_uint4(0xffffffffu, 0u, 0u, 0u);
         if (i0 + lane < cnt) q = __ldg(queue + i0 + lane);
@@ -829,7 +813,7 @@ __global__ void __launch_bounds__(256) k_msssp_push(const uint2 *__restrict__ qu
     const uint64_t first = (uint64_t)wid * per;
     uint32_t p = first < E ? (uint32_t)first : E;
     const uint32_t end = E - p > per ? p + per : E;
-    uint32_t i0 = p < end ? sssp_find(&queue[0].x, 2u, cnt, p) : 0u;
+    uint32_t i0 = p < end ? eg_list_find(&queue[0].x, 2u, cnt, p) : 0u;
     for (; p < end; i0 += 32) {
         uint32_t q_off = 0xffffffffu, q_u = 0, q_j = 0, q_add = 0;
         if (i0 + lane < cnt) {

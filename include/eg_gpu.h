@@ -217,9 +217,9 @@ typedef struct {
      * partitions of 2^k rows (the last candidate) */
     int partition_log2[EG_ROW_SCHEDULES_MAX];
     /* BFS level loop (when the graph has a CSR): mean ms per BFS over 48
-     * sampled roots for the CUDA-graph and the host-driven loop (each at its
-     * best switch divisor of 20, 40, 80, 160, 320), and the form and the
-     * divisor kept for eg_bfs's host_loop = -1 and switch_divisor < 0 */
+     * sampled roots at the best switch divisor of 20, 40, 80, 160, 320 (the
+     * same figure in both fields; bfs_host_loop is 0), and that divisor, kept
+     * for eg_bfs's switch_divisor < 0 */
     float bfs_graph_ms, bfs_host_ms;
     int bfs_host_loop;
     double bfs_switch_divisor; /* the push/pull switch divisor kept */
@@ -287,11 +287,9 @@ typedef struct {
     /* 1: compute parents on the device even when parent_out is NULL (read
      * them later through eg_graph_device_ptr(g, EG_DEV_PARENT)) */
     int device_parents;
-    /* 0: the level loop runs on the device as one CUDA graph with a
-     * conditional while node (no host round trip per level); 1: the host
-     * launches and synchronises every level, each kernel on a grid sized to
-     * its frontier; -1 (default): the form eg_graph_tune found faster on
-     * this graph, else the graph */
+    /* 0, 1 or -1 (default): accepted, all the same.  The level loop is one
+     * cooperative launch with grid barriers between levels; it replaced a
+     * CUDA graph (0) and a loop of launches from the host (1) */
     int host_loop;
 } eg_bfs_opts;
 typedef struct {
