@@ -23,6 +23,7 @@
 //                             per thread as fp32 TwoSum pairs (eg_red2), then
 //                             per CTA in FP64, when REDUCE is set
 #pragma once
+#include <type_traits>
 #include "eg_internal.cuh"
 
 #define EG_MP_NONE 0xffffffffu
@@ -569,6 +570,18 @@ __device__ __forceinline__ void eg_coom_load(const uint32_t *__restrict__ col, c
     }
 }
 
+// The sum of a run's first value: op.first where an op has it (FP64, where
+// adding to zero costs an FP64 instruction), else zero + v.
+template <class Op, class = void>
+struct eg_has_first : std::false_type {};
+template <class Op>
+struct eg_has_first<Op, std::void_t<decltype(&Op::first)>> : std::true_type {};
+template <class Op>
+__device__ __forceinline__ typename Op::A eg_run_start(const Op &op, typename Op::V v) {
+    if constexpr (eg_has_first<Op>::value) return op.first(v);
+    else return op.add(op.zero(), v);
+}
+
 // One warp tile t of the row-id stream (the body of k_coov_rows);
 // `gather(e, u)` returns the value of entry e, source u.  MK: rows from the
 // row-start bits `starts` and the row of every EG_TROW_SPAN-th entry `trow`
@@ -691,7 +704,7 @@ __device__ __forceinline__ void eg_coov_tile(uint32_t t, const uint32_t *__restr
         }
         const uint32_t prev_last = __shfl_up_sync(EG_FULL_MASK, r[U - 1], 1);
         // local runs: head run (from entry 0), middle runs, tail run (to entry U-1)
-        A hsum = op.add(op.zero(), v[0]);
+        A hsum = eg_run_start(op, v[0]);
         A run = hsum;
         bool multi = false;
 #pragma unroll
@@ -700,7 +713,7 @@ __device__ __forceinline__ void eg_coov_tile(uint32_t t, const uint32_t *__restr
                 if (!multi) hsum = run;  // the head run closed at k-1
                 else finish(r[k - 1], run);
                 multi = true;
-                run = op.add(op.zero(), v[k]);
+                run = eg_run_start(op, v[k]);
             } else {
                 run = op.add(run, v[k]);
             }
@@ -722,12 +735,9 @@ __device__ __forceinline__ void eg_coov_tile(uint32_t t, const uint32_t *__restr
         // carry into this lane's head run (multi-run lanes)
         const A prevS = eg_shfl_up(x, 1);
         if (multi) {
-            A tot = hsum;
-            if (lane == 0) {
-                if (r[0] == crow) tot = op.merge(cval, hsum);
-            } else if (prev_last == r[0]) {
-                tot = op.merge(prevS, hsum);
-            }
+            const bool on = lane == 0 ? r[0] == crow : prev_last == r[0];
+            A tot = lane == 0 ? cval : prevS;
+            tot = on ? op.merge(tot, hsum) : hsum;
             finish(r[0], tot);
         }
         if (nxt != r[U - 1]) finish(r[U - 1], x);
