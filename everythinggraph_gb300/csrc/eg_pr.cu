@@ -266,6 +266,15 @@ __global__ void k_pr_reduce(const double2 *__restrict__ part, uint32_t nparts, e
 #define EG_PR_CHECK 4  // iterations between reads of the stop flag
 #define EG_PR_RES_BLOCKS 1024
 #define EG_ROW_CFGS 12
+// Warps per SM up to which the default schedule keeps tiles short (128, 256,
+// 512 entries, then 1024): more warps in flight on small graphs, several waves
+// that even out on middle ones.  SpMV row passes, all tiles 1024 -> this rule:
+// RMAT m = 100K 21 -> 17 us (fp64 29 -> 21), m = 1.6M 25 -> 23 (37 -> 30),
+// m = 6.4M 47 -> 43 (75 -> 64), m = 13M 67 -> 63 (106 -> 97); with 640, 128
+// entries at m = 13M: 75 us.  PageRank m = 3M 18.3 -> 12.9 us, m = 20M
+// 64 -> 60 us; with block sums per CTA (tolerance, dangling mass) longer tiles
+// stay better: m = 12M 52 us at 1024, 55 at 512.
+#define EG_COO_FILL 320
 struct RowCfg {
     int tile, u, pf, minb, hint;
 };
@@ -277,6 +286,13 @@ static const RowCfg kRowCfg[EG_ROW_CFGS] = {
     {1024, 4, 1, 5, 0}, {2048, 4, 0, 6, 0}, {2048, 4, 1, 5, 0}, {1024, 4, 1, 6, 0}, {512, 4, 1, 5, 0},
     {1024, 8, 1, 4, 0}, {1024, 4, 0, 8, 0}, {2048, 8, 0, 5, 0}, {1024, 4, 1, 5, 1}, {2048, 4, 1, 5, 1},
     {1024, 4, 2, 4, 0}, {2048, 4, 2, 4, 0}};
+
+// SpMV's ops: the default schedule (0) keeps the streamed row ids and columns
+// out of L1 and first in line for L2 eviction, which leaves L2 to x: uniform
+// n = 2^25, m = 2^30 (x twice an L2 half) 5.06 -> 4.65 ms, RMAT n = 2^25,
+// m = 2^29 2.13 -> 2.09 ms; x within L2: no difference.
+template <class Op>
+struct coo_spmv : std::false_type {};
 
 template <class Op, int TILE, int U, bool REDUCE, int PF, int MINB, int HINT = 0, bool MK = false>
 static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part, const Op &op, uint32_t *nparts,
@@ -349,9 +365,26 @@ static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part
         EG_ROW_CASE(10, 1024, 4, 2, 4, 0)
         EG_ROW_CASE(11, 2048, 4, 2, 4, 0)
         default:
-            return coo_launch_t<Op, 1024, 4, REDUCE, true, 5, 0, MK>(g, adj, carry_buf, part, op, nparts, ev_begin,
-                                                                     ev_end, m_entries, empty_rows, empty_from);
+            break;
     }
+    const uint64_t entries = m_entries == EG_ALL_ENTRIES ? g->m : m_entries;
+    constexpr bool SPMV = coo_spmv<Op>::value;
+    constexpr int H = SPMV ? 1 : 0;
+    const uint64_t warps = (uint64_t)g->ctx->sm_count * EG_COO_FILL;
+#define EG_ROW_TILE(T, PF)                                                                                    \
+    if (entries <= T * warps)                                                                                  \
+        return coo_launch_t<Op, T, 4, REDUCE, PF, 5, H, MK>(g, adj, carry_buf, part, op, nparts, ev_begin, ev_end, \
+                                                            m_entries, empty_rows, empty_from);
+    if constexpr (SPMV) {
+        EG_ROW_TILE(128, 0)
+        EG_ROW_TILE(256, 1)
+    }
+    if constexpr (SPMV || (MK && !REDUCE)) {
+        EG_ROW_TILE(512, 1)
+    }
+    return coo_launch_t<Op, 1024, 4, REDUCE, 1, 5, H, MK>(g, adj, carry_buf, part, op, nparts, ev_begin, ev_end,
+                                                          m_entries, empty_rows, empty_from);
+#undef EG_ROW_TILE
 #undef EG_ROW_CASE
 }
 
@@ -1019,6 +1052,13 @@ struct SpmvF64Op {
         return make_float2(0.f, 0.f);
     }
 };
+
+template <int MODE>
+struct coo_spmv<SpmvU32Op<MODE>> : std::true_type {};
+template <bool COMP>
+struct coo_spmv<SpmvF32Op<COMP>> : std::true_type {};
+template <>
+struct coo_spmv<SpmvF64Op> : std::true_type {};
 
 // Edge value of CSC entry p (row v, column u): U[0,1) hashed from the
 // unordered endpoint pair, or 1.
