@@ -283,11 +283,12 @@ __host__ __device__ __forceinline__ uint64_t eg_edge_hash(uint64_t seed, uint32_
 }
 
 // Two running sums (e.g. a residual and a dangling mass) kept by one thread
-// as fp32 (sum, error) pairs (Knuth's TwoSum) and widened to FP64 once per
-// thread before the FP64 block reduction.  FP64 instructions issue at a small
-// fraction of the fp32 rate on this GPU, and per-row sums often run in
-// divergent code (one lane per finished row), so per-row FP64 adds would
-// dominate the kernels that carry them.
+// as fp32 (sum, error) pairs (Knuth's TwoSum), summed over the block in the
+// same form and widened to FP64 once per block.  FP64 instructions issue at a
+// small fraction of the fp32 rate on this GPU: per-row FP64 adds, often in
+// divergent code, would dominate the kernels that carry them, and FP64 sums
+// per warp cost PageRank's row pass over 12M entries 3 of its 51 us, the L1
+// change of 4M ranks 7 of its 13.
 struct eg_red2 {
     float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f;
     __device__ __forceinline__ static void two_sum(float &s, float &c, float x) {
@@ -303,7 +304,39 @@ struct eg_red2 {
     __device__ __forceinline__ double2 wide() const {
         return make_double2((double)s0 + (double)c0, (double)s1 + (double)c1);
     }
+    __device__ __forceinline__ float4 pack() const { return make_float4(s0, c0, s1, c1); }
+    __device__ __forceinline__ static eg_red2 unpack(float4 x) {
+        eg_red2 r;
+        r.s0 = x.x;
+        r.c0 = x.y;
+        r.s1 = x.z;
+        r.c1 = x.w;
+        return r;
+    }
 };
+// A warp's sums in its lane 0.
+__device__ __forceinline__ eg_red2 eg_warp_sum(eg_red2 acc) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float s0 = __shfl_down_sync(0xffffffffu, acc.s0, o), c0 = __shfl_down_sync(0xffffffffu, acc.c0, o);
+        const float s1 = __shfl_down_sync(0xffffffffu, acc.s1, o), c1 = __shfl_down_sync(0xffffffffu, acc.c1, o);
+        acc.add(make_float2(s0, s1));
+        acc.c0 += c0;
+        acc.c1 += c1;
+    }
+    return acc;
+}
+// The block's sums in thread 0 (whole warps; s_sum: 32 entries).
+__device__ __forceinline__ eg_red2 eg_block_sum(eg_red2 acc, float4 *s_sum) {
+    acc = eg_warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc.pack();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        acc = threadIdx.x < (blockDim.x >> 5) ? eg_red2::unpack(s_sum[threadIdx.x]) : eg_red2();
+        acc = eg_warp_sum(acc);
+    }
+    return acc;
+}
 
 // SSSP edge weights computed from the endpoints (no weight array), and the
 // extension of a path distance by one edge in the rule's encoding: u32 sums

@@ -315,49 +315,27 @@ struct eg_f2sum {
 // Entries carry their row id (rid[e], the COO form of the CSR/CSC, built once
 // per graph), so a warp can own a fixed range of entries and find row
 // boundaries by comparing neighbouring row ids.  Rows split between warps are
-// finished by k_coo_fixup (same head/tail scheme as the merge-path kernels);
-// rows without entries are written by k_coo_empty_rows (or, when they are
-// known to form the range at the end, k_coo_empty_range).
+// finished by k_coo_tail (same head/tail scheme as the merge-path kernels),
+// which also writes the rows without entries.
 
 // The block's share of the emitted (residual, dangling) partials into part[blockIdx.x].
 template <bool REDUCE>
-__device__ __forceinline__ void eg_block_part(const eg_red2 &redf, double2 *__restrict__ part, double2 *s_red) {
+__device__ __forceinline__ void eg_block_part(const eg_red2 &redf, float4 *__restrict__ part, float4 *s_red) {
     if (!REDUCE) return;
-    double2 red = redf.wide();
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        red.x += __shfl_down_sync(EG_FULL_MASK, red.x, o);
-        red.y += __shfl_down_sync(EG_FULL_MASK, red.y, o);
-    }
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = red;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 t = make_double2(0.0, 0.0);
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-            t.x += s_red[w].x;
-            t.y += s_red[w].y;
-        }
-        part[blockIdx.x] = t;
-    }
+    const eg_red2 sum = eg_block_sum(redf, s_red);
+    if (threadIdx.x == 0) part[blockIdx.x] = sum.pack();
 }
 
 // Rows split between warp tiles, finished from the tiles' head and tail
-// partials: one thread per tile.  A head row that began in the tile before
-// is finished by the tile's thread (that tile's tail + this tile's head);
-// a row spanning more tiles is finished by the whole warp, which adds the
-// tails of the preceding tiles 32 per step.  Both give the same bits (the
-// tail and head are merged in that order either way).
+// partials: one thread per tile c.  A head row that began in the tile before
+// is finished by the tile's thread (that tile's tail + this tile's head); a
+// row over more tiles by the whole warp, every 32nd tail per lane.
 template <class Op, int TILE_E, bool REDUCE>
-__global__ void k_coo_fixup(const uint32_t *__restrict__ ptr, uint32_t ntiles,
-                            const eg_mp_carry<typename Op::A> *__restrict__ carry, double2 *__restrict__ part,
-                            Op op) {
+__device__ __forceinline__ void eg_coo_fixup(uint32_t c, const uint32_t *__restrict__ ptr, uint32_t ntiles,
+                                             const eg_mp_carry<typename Op::A> *__restrict__ carry, const Op &op,
+                                             eg_red2 &redf) {
     using A = typename Op::A;
-    __shared__ double2 s_red[32];
-    if (!op.active()) return;
-    op.setup();
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    eg_red2 redf;
     uint32_t row = EG_MP_NONE, rstart = 0;
     bool wide = false;
     if (c < ntiles) {
@@ -378,42 +356,29 @@ __global__ void k_coo_fixup(const uint32_t *__restrict__ ptr, uint32_t ntiles,
         todo &= todo - 1;
         const uint32_t cw = __shfl_sync(EG_FULL_MASK, c, src);
         const uint32_t rw = __shfl_sync(EG_FULL_MASK, row, src);
-        const uint32_t sw = __shfl_sync(EG_FULL_MASK, rstart, src);
-        A tot = carry[cw].head_val;
-        for (int base = (int)cw - 1; base >= 0; base -= 32) {
-            const int k = base - (int)lane;
-            const bool valid = k >= 0;
-            const bool began = valid && sw >= (uint32_t)k * (uint32_t)TILE_E;
-            const uint32_t stop_mask = __ballot_sync(EG_FULL_MASK, began || !valid);
-            const int last = stop_mask ? __ffs(stop_mask) - 1 : 31;
-            A x = (valid && (int)lane <= last) ? carry[k].tail_val : op.zero();
+        const uint32_t first = __shfl_sync(EG_FULL_MASK, rstart, src) / (uint32_t)TILE_E;  // where the row began
+        A x = op.zero();
+#pragma unroll 4
+        for (uint32_t k = first + lane; k < cw; k += 32) x = op.merge(x, carry[k].tail_val);
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const A y = eg_shfl_down(x, off);
-                x = op.merge(y, x);
-            }
-            x = eg_shfl_idx(x, 0);
-            tot = op.merge(x, tot);
-            if (stop_mask) break;
+        for (int off = 16; off > 0; off >>= 1) {
+            const A y = eg_shfl_down(x, off);
+            x = op.merge(x, y);
         }
-        if ((int)lane == src) {
-            const float2 d = op.emit(rw, tot);
+        if (lane == 0) {
+            const float2 d = op.emit(rw, op.merge(x, carry[cw].head_val));
             if (REDUCE) redf.add(d);
         }
     }
-    eg_block_part<REDUCE>(redf, part, s_red);
 }
 
 // Rows without entries: emitted with an empty sum.  Four rows per thread and
-// step, their row pointers loaded before any is tested.
+// step, their row pointers loaded before any is tested.  Block b of nb.
 template <class Op, bool REDUCE>
-__global__ void k_coo_empty_rows(const uint32_t *__restrict__ ptr, uint32_t n, double2 *__restrict__ part, Op op) {
-    __shared__ double2 s_red[32];
-    if (!op.active()) return;
-    op.setup();
-    eg_red2 redf;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v0 < n; v0 += 4 * stride) {
+__device__ __forceinline__ void eg_coo_empty_rows(uint32_t b, uint32_t nb, const uint32_t *__restrict__ ptr,
+                                                  uint32_t n, const Op &op, eg_red2 &redf) {
+    const uint64_t stride = (uint64_t)nb * blockDim.x;
+    for (uint64_t v0 = (uint64_t)b * blockDim.x + threadIdx.x; v0 < n; v0 += 4 * stride) {
         uint32_t lo[4], hi[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -433,22 +398,63 @@ __global__ void k_coo_empty_rows(const uint32_t *__restrict__ ptr, uint32_t n, d
             }
         }
     }
-    eg_block_part<REDUCE>(redf, part, s_red);
 }
 
 // Rows [lo, hi), known to have no entries (the relabelled CSC keeps them
-// last): emitted with an empty sum, without reading row pointers.
+// last): emitted with an empty sum, without reading row pointers; what each
+// emit reads of its row (Op::load) four rows ahead of the first store.
 template <class Op, bool REDUCE>
-__global__ void k_coo_empty_range(uint32_t lo, uint32_t hi, double2 *__restrict__ part, Op op) {
-    __shared__ double2 s_red[32];
+__device__ __forceinline__ void eg_coo_empty_range(uint32_t b, uint32_t nb, uint32_t lo, uint32_t hi, const Op &op,
+                                                   eg_red2 &redf) {
+    const uint64_t stride = (uint64_t)nb * blockDim.x;
+    for (uint64_t v0 = (uint64_t)lo + (uint64_t)b * blockDim.x + threadIdx.x; v0 < hi; v0 += 4 * stride) {
+        uint32_t x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] = v0 + j * stride < hi ? op.load((uint32_t)(v0 + j * stride)) : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (v0 + j * stride >= hi) break;
+            const float2 d = op.emit((uint32_t)(v0 + j * stride), op.zero(), x[j]);
+            if (REDUCE) redf.add(d);
+        }
+    }
+}
+
+// What is left after the row kernel, in one launch: blocks 0 .. gf - 1 finish
+// the rows split between tiles, the others write the rows without entries
+// (EMPTY 1: by the row pointers, 2: the range [empty_from, n)).  Bound by
+// chains of dependent loads.  PageRank on RMAT n = 4M, m = 40M with dangling
+// mass: 26 us as two launches -> 9; n = 300K, m = 3M 7.6 -> 4.9 us (long rows
+// spread over the warps).
+template <class Op, int TILE_E, bool REDUCE, int EMPTY>
+__global__ void k_coo_tail(const uint32_t *__restrict__ ptr, uint32_t n, uint32_t empty_from, uint32_t ntiles,
+                           uint32_t gf, const eg_mp_carry<typename Op::A> *__restrict__ carry,
+                           float4 *__restrict__ part, Op op) {
+    __shared__ float4 s_red[32];
     if (!op.active()) return;
     op.setup();
     eg_red2 redf;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t v = (uint64_t)lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < hi; v += stride) {
-        const float2 d = op.emit((uint32_t)v, op.zero());
-        if (REDUCE) redf.add(d);
+    const uint32_t b = blockIdx.x;
+    if (b < gf) {
+        // neighbouring tiles in different warps: long rows come in groups
+        const uint32_t warps = gf * (blockDim.x >> 5), w = (b * blockDim.x + threadIdx.x) >> 5;
+        eg_coo_fixup<Op, TILE_E, REDUCE>((threadIdx.x & 31) * warps + w, ptr, ntiles, carry, op, redf);
+    } else if constexpr (EMPTY == 1) {
+        eg_coo_empty_rows<Op, REDUCE>(b - gf, gridDim.x - gf, ptr, n, op, redf);
+    } else if constexpr (EMPTY == 2) {
+        eg_coo_empty_range<Op, REDUCE>(b - gf, gridDim.x - gf, empty_from, n, op, redf);
     }
+    eg_block_part<REDUCE>(redf, part, s_red);
+}
+
+// The range alone (layouts whose row kernel splits no rows).
+template <class Op, bool REDUCE>
+__global__ void k_coo_empty_range(uint32_t lo, uint32_t hi, float4 *__restrict__ part, Op op) {
+    __shared__ float4 s_red[32];
+    if (!op.active()) return;
+    op.setup();
+    eg_red2 redf;
+    eg_coo_empty_range<Op, REDUCE>(blockIdx.x, gridDim.x, lo, hi, op, redf);
     eg_block_part<REDUCE>(redf, part, s_red);
 }
 
@@ -504,27 +510,6 @@ __device__ __forceinline__ void eg_coov_load(const uint32_t *__restrict__ rid, c
             r[k] = in ? __ldg(rid + e + k) : EG_MP_NONE;
             u[k] = in ? __ldg(col + e + k) : 0u;
         }
-    }
-}
-
-// Block sum of the emitted (residual, dangling) pairs into part[blockIdx.x].
-__device__ __forceinline__ void eg_coov_reduce(const eg_red2 &redf, double2 *s_red, uint32_t nwarps,
-                                               double2 *__restrict__ part) {
-    double2 red = redf.wide();
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        red.x += __shfl_down_sync(EG_FULL_MASK, red.x, o);
-        red.y += __shfl_down_sync(EG_FULL_MASK, red.y, o);
-    }
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = red;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 sum = make_double2(0.0, 0.0);
-        for (uint32_t w = 0; w < nwarps; w++) {
-            sum.x += s_red[w].x;
-            sum.y += s_red[w].y;
-        }
-        part[blockIdx.x] = sum;
     }
 }
 
@@ -781,13 +766,13 @@ template <class Op, int TILE_E, int U, bool REDUCE, int PF = 0, int MINB = 6, in
 __global__ void __launch_bounds__(256, MINB) k_coov_rows(const uint32_t *__restrict__ rid,
                                                          const uint32_t *__restrict__ col, uint32_t m, uint32_t ntiles,
                                                          eg_mp_carry<typename Op::A> *__restrict__ carry,
-                                                         double2 *__restrict__ part, Op op,
+                                                         float4 *__restrict__ part, Op op,
                                                          const uint32_t *__restrict__ starts = nullptr,
                                                          const uint32_t *__restrict__ trow = nullptr) {
     static_assert(U == 4 || U == 8, "4 or 8 entries per lane");
     static_assert(TILE_E % (32 * U) == 0, "tiles hold whole chunks");
     static_assert(!MK || TILE_E % EG_TROW_SPAN == 0, "tiles start at a row sample");
-    __shared__ double2 s_red[8];
+    __shared__ float4 s_red[32];
     if (!op.active()) return;
     op.setup();
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -797,5 +782,5 @@ __global__ void __launch_bounds__(256, MINB) k_coov_rows(const uint32_t *__restr
         eg_coov_tile<Op, TILE_E, U, REDUCE, PF, HINT, MK>(
             t, rid, col, starts, trow, m, carry, op, redf, [&](uint32_t e, uint32_t u) { return op.gather(e, u); },
             pol);
-    if (REDUCE) eg_coov_reduce(redf, s_red, 8, part);
+    eg_block_part<REDUCE>(redf, part, s_red);
 }

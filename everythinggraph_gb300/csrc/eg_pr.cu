@@ -16,7 +16,7 @@
 //   k_coov_rows<PrOp>      rank[v] = base + d * sum_{u in in(v)} contrib[u],
 //                          contrib'[v] = rank[v] / deg[v] (fused into the write);
 //                          warp tiles of row-id/column pairs (eg_mp.cuh)
-//   k_coo_empty_range, k_coo_fixup  rows without entries, rows split between tiles
+//   k_coo_tail             rows split between tiles, rows without entries
 //   k_pr_residual          (with a tolerance) the L1 change, coalesced
 //   k_pr_reduce            FP64 residual / dangling mass -> next base, stop flag
 // On small graphs all iterations are one cooperative launch (eg_prsmall.cuh).
@@ -106,7 +106,9 @@ struct PrOp {
         if constexpr (COMP) return eg_f2sum::merge(a, b);
         else return a + b;
     }
-    __device__ __forceinline__ float2 emit(uint32_t v, A s) const {
+    __device__ __forceinline__ uint32_t load(uint32_t v) const { return deg[v]; }
+    __device__ __forceinline__ float2 emit(uint32_t v, A s) const { return emit(v, s, load(v)); }
+    __device__ __forceinline__ float2 emit(uint32_t v, A s, uint32_t deg_v) const {
         float sum;
         if constexpr (COMP) sum = s.x + s.y;
         else sum = s;
@@ -115,7 +117,7 @@ struct PrOp {
         const float b = seeds.count ? base * seeds.weight(v) : base;
         float r = fmaf(damping, sum, b);
         rank[v] = r;
-        uint32_t d = deg[v] * mult;
+        uint32_t d = deg_v * mult;
         cout[v] = d ? __fdiv_rn(r, (float)d) : 0.f;
         return make_float2(0.f, d ? 0.f : r);  // (residual: k_pr_residual, dangling mass)
     }
@@ -144,65 +146,54 @@ struct PrAccOp {
 
 // rank = prev_init, contrib = prev_init / deg; partial dangling mass
 __global__ void k_pr_init(uint32_t n, float prev_init, const uint32_t *__restrict__ deg, uint32_t mult,
-                          float *__restrict__ rank, float *__restrict__ contrib, double2 *__restrict__ part) {
-    __shared__ double s_red[8];
-    double dang = 0.0;
+                          float *__restrict__ rank, float *__restrict__ contrib, float4 *__restrict__ part) {
+    __shared__ float4 s_red[32];
+    eg_red2 dang;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         uint32_t d = deg[v] * mult;
         rank[v] = prev_init;
         contrib[v] = d ? __fdiv_rn(prev_init, (float)d) : 0.f;
-        if (!d) dang += (double)prev_init;
+        if (!d) dang.add(make_float2(0.f, prev_init));
     }
-    for (int o = 16; o > 0; o >>= 1) dang += __shfl_down_sync(EG_FULL_MASK, dang, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = dang;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += s_red[w];
-        part[blockIdx.x] = make_double2(0.0, s);
-    }
+    dang = eg_block_sum(dang, s_red);
+    if (threadIdx.x == 0) part[blockIdx.x] = dang.pack();
 }
 
 // Personalised start vector: multiplicity / total seeds on the seeds, 0 elsewhere.
 __global__ void k_ppr1_init(uint32_t n, PprSeeds seeds, float inv_total, const uint32_t *__restrict__ deg,
-                            float *__restrict__ rank, float *__restrict__ contrib, double2 *__restrict__ part) {
-    __shared__ double s_red[8];
-    double dang = 0.0;
+                            float *__restrict__ rank, float *__restrict__ contrib, float4 *__restrict__ part) {
+    __shared__ float4 s_red[32];
+    eg_red2 dang;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const uint32_t d = deg[v];
         const float r = seeds.weight(v) * inv_total;
         rank[v] = r;
         contrib[v] = d ? __fdiv_rn(r, (float)d) : 0.f;
-        if (!d) dang += (double)r;
+        if (!d) dang.add(make_float2(0.f, r));
     }
-    for (int o = 16; o > 0; o >>= 1) dang += __shfl_down_sync(EG_FULL_MASK, dang, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = dang;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_red[w];
-        part[blockIdx.x] = make_double2(0.0, t);
-    }
+    dang = eg_block_sum(dang, s_red);
+    if (threadIdx.x == 0) part[blockIdx.x] = dang.pack();
 }
 
-// L1 change between two rank vectors, per-block FP64 partials in .x (the
+// L1 change between two rank vectors, per-block partials in the first sum (the
 // stop test's residual); skipped once the run has converged.
 __global__ void k_pr_residual(const float *__restrict__ cur, const float *__restrict__ prev, uint32_t n,
-                              const eg_pr_dev *st, double2 *__restrict__ part) {
-    __shared__ double s_red[8];
+                              const eg_pr_dev *st, float4 *__restrict__ part) {
+    __shared__ float4 s_red[32];
     if (st->done) return;
     eg_red2 acc;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        acc.add(make_float2(fabsf(__ldg(cur + v) - __ldg(prev + v)), 0.f));
-    double r = acc.wide().x;
-    for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(EG_FULL_MASK, r, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = r;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_red[w];
-        part[blockIdx.x] = make_double2(t, 0.0);
+    const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);  // 16 bytes per load (the arrays' ends are padded)
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        const float4 c = __ldg(reinterpret_cast<const float4 *>(cur) + q);
+        const float4 p = __ldg(reinterpret_cast<const float4 *>(prev) + q);
+        const uint32_t left = n - 4 * q;  // past the end: no change
+        const float d[4] = {fabsf(c.x - p.x), left > 1 ? fabsf(c.y - p.y) : 0.f, left > 2 ? fabsf(c.z - p.z) : 0.f,
+                            left > 3 ? fabsf(c.w - p.w) : 0.f};
+#pragma unroll
+        for (int k = 0; k < 4; k++) eg_red2::two_sum(acc.s0, acc.c0, d[k]);
     }
+    acc = eg_block_sum(acc, s_red);
+    if (threadIdx.x == 0) part[blockIdx.x] = acc.pack();
 }
 
 __global__ void k_map_ids(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ in, uint32_t k,
@@ -220,27 +211,25 @@ __global__ void k_pr_unpermute(const float *__restrict__ rank_a, const float *__
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) rank[v] = src[perm[v]];
 }
 
-// One block: deterministic FP64 sum of the partials, next base, stop test.
-__global__ void k_pr_reduce(const double2 *__restrict__ part, uint32_t nparts, eg_pr_dev *st, double tele_div,
+// One block: deterministic sum of the partials, widened to FP64 at the end;
+// next base, stop test.  fp32 pairs: 7.0 us for 6.2K partials and 2.1 for none,
+// 15.4 and 3.2 as FP64 sums.
+#define EG_PR_RED_T 512
+__global__ void k_pr_reduce(const float4 *__restrict__ part, uint32_t nparts, eg_pr_dev *st, double tele_div,
                             float damping, int dangling, double tol, int count_iter) {
-    __shared__ double2 s[256];
+    __shared__ float4 s[32];
     if (st->done) return;
-    double2 acc = make_double2(0.0, 0.0);
-    for (uint32_t i = threadIdx.x; i < nparts; i += blockDim.x) {
-        acc.x += part[i].x;
-        acc.y += part[i].y;
+    eg_red2 acc;
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < nparts; i += EG_PR_RED_T) {
+        const float4 p = part[i];
+        acc.add(make_float2(p.x, p.z));
+        acc.c0 += p.y;
+        acc.c1 += p.w;
     }
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            s[threadIdx.x].x += s[threadIdx.x + w].x;
-            s[threadIdx.x].y += s[threadIdx.x + w].y;
-        }
-        __syncthreads();
-    }
+    if (nparts) acc = eg_block_sum(acc, s);
     if (threadIdx.x == 0) {
-        double res = s[0].x, dang = s[0].y;
+        const double res = acc.wide().x, dang = acc.wide().y;
         st->residual = res;
         st->dangling = dang;
         double b = (1.0 - (double)damping) / tele_div;
@@ -272,8 +261,8 @@ __global__ void k_pr_reduce(const double2 *__restrict__ part, uint32_t nparts, e
 // RMAT m = 100K 21 -> 17 us (fp64 29 -> 21), m = 1.6M 25 -> 23 (37 -> 30),
 // m = 6.4M 47 -> 43 (75 -> 64), m = 13M 67 -> 63 (106 -> 97); with 640, 128
 // entries at m = 13M: 75 us.  PageRank m = 3M 18.3 -> 12.9 us, m = 20M
-// 64 -> 60 us; with block sums per CTA (tolerance, dangling mass) longer tiles
-// stay better: m = 12M 52 us at 1024, 55 at 512.
+// 64 -> 60 us; with sums per CTA (tolerance, dangling mass) it depends on the
+// graph: uniform m = 12M 48 us at 1024, 50 at 512, RMAT m = 14M 39.7 and 38.2.
 #define EG_COO_FILL 320
 struct RowCfg {
     int tile, u, pf, minb, hint;
@@ -295,7 +284,7 @@ template <class Op>
 struct coo_spmv : std::false_type {};
 
 template <class Op, int TILE, int U, bool REDUCE, int PF, int MINB, int HINT = 0, bool MK = false>
-static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part, const Op &op, uint32_t *nparts,
+static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *part, const Op &op, uint32_t *nparts,
                         cudaEvent_t ev_begin, cudaEvent_t ev_end, uint64_t m_entries, bool empty_rows,
                         uint32_t empty_from) {
     static_assert(!MK || TILE % EG_TROW_SPAN == 0, "masked tiles start at a row sample");
@@ -322,18 +311,19 @@ static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *pa
         EG_LAUNCHED(ctx);
         if (ev_end) EG_CUDA(cudaEventRecord(ev_end, ctx->stream));
     }
-    if (g2 && ranged) {
-        k_coo_empty_range<Op, REDUCE><<<g2, 256, 0, ctx->stream>>>(empty_from, g->n, part ? part + g1_parts : nullptr,
-                                                                   op);
-        EG_LAUNCHED(ctx);
-    } else if (g2) {
-        k_coo_empty_rows<Op, REDUCE><<<g2, 256, 0, ctx->stream>>>(bp<uint32_t>(adj.ptr), g->n,
-                                                                  part ? part + g1_parts : nullptr, op);
-        EG_LAUNCHED(ctx);
-    }
-    if (gf) {
-        k_coo_fixup<Op, TILE, REDUCE><<<gf, 256, 0, ctx->stream>>>(
-            bp<uint32_t>(adj.ptr), ntiles, bp<eg_mp_carry<A>>(carry_buf), part ? part + g1_parts + g2 : nullptr, op);
+    if (g2 + gf) {
+        const auto *carry = bp<eg_mp_carry<A>>(carry_buf);
+        float4 *tail = part ? part + g1_parts : nullptr;
+        const uint32_t *ptr = bp<uint32_t>(adj.ptr);
+        if constexpr (MK) {
+            if (!ranged) return eg_fail(EG_EINVAL, "masked rows without an empty range");
+            k_coo_tail<Op, TILE, REDUCE, 2><<<gf + g2, 256, 0, ctx->stream>>>(ptr, g->n, empty_from, ntiles, gf, carry,
+                                                                               tail, op);
+        } else {
+            if (ranged) return eg_fail(EG_EINVAL, "an empty range without masked rows");
+            k_coo_tail<Op, TILE, REDUCE, 1><<<gf + g2, 256, 0, ctx->stream>>>(ptr, g->n, 0u, ntiles, gf, carry, tail,
+                                                                               op);
+        }
         EG_LAUNCHED(ctx);
     }
     *nparts = g1_parts + g2 + gf;
@@ -345,7 +335,7 @@ static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *pa
 // empty_from <= n: the rows without entries are exactly [empty_from, n).
 // MK: `adj` is the relabelled CSC, read through its row-start bits.
 template <class Op, bool REDUCE, bool MK = false>
-static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part, const Op &op, uint32_t *nparts,
+static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *part, const Op &op, uint32_t *nparts,
                       cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr,
                       uint64_t m_entries = EG_ALL_ENTRIES, bool empty_rows = true, uint32_t empty_from = EG_NO_RANGE) {
 #define EG_ROW_CASE(i, T, U, PF, MB, H)                                                                             \
@@ -379,7 +369,7 @@ static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part
         EG_ROW_TILE(128, 0)
         EG_ROW_TILE(256, 1)
     }
-    if constexpr (SPMV || (MK && !REDUCE)) {
+        if constexpr (SPMV || (MK && !REDUCE)) {
         EG_ROW_TILE(512, 1)
     }
     return coo_launch_t<Op, 1024, 4, REDUCE, 1, 5, H, MK>(g, adj, carry_buf, part, op, nparts, ev_begin, ev_end,
@@ -402,7 +392,7 @@ static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, double2 *part
 #endif
 #define EG_PR_CANDS (EG_ROW_CFGS + 1)  // the tuner's candidates: the row schedules, then the partition kernel
 template <bool REDUCE>
-static int pcol_launch(eg_graph *g, const PrOp<false> &op, double2 *part, uint32_t *nparts, cudaEvent_t ev_begin,
+static int pcol_launch(eg_graph *g, const PrOp<false> &op, float4 *part, uint32_t *nparts, cudaEvent_t ev_begin,
                        cudaEvent_t ev_end, bool empty_rows, double mass) {
     eg_ctx *ctx = g->ctx;
     eg_pcols &pc = g->pcol;
@@ -492,7 +482,7 @@ static uint32_t pr_block_log2(const eg_graph *g, const eg_pr_opts &o) {
 // EG_KEV iterations are bracketed by the context's kernel events.
 template <bool COMP, bool REDUCE>
 static int pr_iterations(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, double tele_div, eg_pr_dev *st,
-                         double2 *part, eg_buf &carry, bool timed, int it0, int it1) {
+                         float4 *part, eg_buf &carry, bool timed, int it0, int it1) {
     eg_ctx *ctx = g->ctx;
     for (int it = it0; it < it1; it++) {
         PrOp<COMP> op;
@@ -565,7 +555,7 @@ static int pr_iterations(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, d
             EG_LAUNCHED(ctx);
             nparts += EG_PR_RES_BLOCKS;
         }
-        k_pr_reduce<<<1, 256, 0, ctx->stream>>>(part, REDUCE ? nparts : 0, st, tele_div, o.damping, o.dangling,
+        k_pr_reduce<<<1, EG_PR_RED_T, 0, ctx->stream>>>(part, REDUCE ? nparts : 0, st, tele_div, o.damping, o.dangling,
                                                 o.tolerance, 1);
         EG_LAUNCHED(ctx);
     }
@@ -574,7 +564,7 @@ static int pr_iterations(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, d
 
 // Iterations [it0, it1).
 static int pr_dispatch(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, double tele_div, bool reduce,
-                       eg_pr_dev *st, double2 *part, eg_buf &carry, bool timed, int it0, int it1) {
+                       eg_pr_dev *st, float4 *part, eg_buf &carry, bool timed, int it0, int it1) {
     if (o.compensated) {
         if (reduce) return pr_iterations<true, true>(g, o, ps, tele_div, st, part, carry, timed, it0, it1);
         return pr_iterations<true, false>(g, o, ps, tele_div, st, part, carry, timed, it0, it1);
@@ -585,7 +575,7 @@ static int pr_dispatch(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, dou
 
 // The iteration loop of plain PageRank captured once as a CUDA graph and
 // replayed while the options and the buffers it was captured with stay the same.
-static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st, double2 *part, eg_buf &carry) {
+static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st, float4 *part, eg_buf &carry) {
     eg_ctx *ctx = g->ctx;
     uint64_t key[16] = {};
     key[0] = (uint32_t)o.iterations | ((uint64_t)g->csc_p_rows << 32);
@@ -699,12 +689,12 @@ static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t
     EG_TRY(eg_buf_ensure(ctx, g->rank_q, (uint64_t)n * 4));
     EG_TRY(eg_buf_ensure(ctx, g->contrib0, (uint64_t)n * 4));
     EG_TRY(eg_buf_ensure(ctx, g->contrib1, (uint64_t)n * 4));
-    EG_TRY(eg_buf_ensure(ctx, g->pr_part, ((uint64_t)nparts + 1024) * sizeof(double2)));
+    EG_TRY(eg_buf_ensure(ctx, g->pr_part, ((uint64_t)nparts + 1024) * sizeof(float4)));
     eg_buf &carry = g->mp_carry;
     eg_pr_dev *st = bp<eg_pr_dev>(g->pr_stats);
-    double2 *part = bp<double2>(g->pr_part);
+    float4 *part = bp<float4>(g->pr_part);
     EG_CUDA(cudaMemsetAsync(st, 0, sizeof(eg_pr_dev), ctx->stream));
-    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(double2), ctx->stream));
+    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(float4), ctx->stream));
     const bool ppr = ps.count > 0;
     const double tele_div = ppr ? (double)seed_total : (double)n;
     const bool reduce = o.tolerance > 0.0 || o.dangling;
@@ -719,9 +709,9 @@ static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t
                                               bp<float>(g->rank_p), bp<float>(g->contrib0), part);
     }
     EG_LAUNCHED(ctx);
-    k_pr_reduce<<<1, 256, 0, ctx->stream>>>(part, ib, st, tele_div, o.damping, o.dangling, 0.0, 0);
+    k_pr_reduce<<<1, EG_PR_RED_T, 0, ctx->stream>>>(part, ib, st, tele_div, o.damping, o.dangling, 0.0, 0);
     EG_LAUNCHED(ctx);
-    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(double2), ctx->stream));
+    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(float4), ctx->stream));
     const bool graph = o.use_graph && !ppr;
     if (graph) EG_TRY(pr_graph(g, o, reduce, st, part, carry));
     EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));

@@ -70,35 +70,10 @@ __device__ __forceinline__ uint32_t prs_rows_below(const uint32_t *__restrict__ 
     return lo;
 }
 
-// A warp's sums in its lane 0.
-__device__ __forceinline__ eg_red2 prs_warp_sum(eg_red2 acc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float s0 = __shfl_down_sync(EG_FULL_MASK, acc.s0, o), c0 = __shfl_down_sync(EG_FULL_MASK, acc.c0, o);
-        const float s1 = __shfl_down_sync(EG_FULL_MASK, acc.s1, o), c1 = __shfl_down_sync(EG_FULL_MASK, acc.c1, o);
-        acc.add(make_float2(s0, s1));
-        acc.c0 += c0;
-        acc.c1 += c1;
-    }
-    return acc;
-}
-__device__ __forceinline__ eg_red2 prs_unpack(float4 x) {
-    eg_red2 r;
-    r.s0 = x.x;
-    r.c0 = x.y;
-    r.s1 = x.z;
-    r.c1 = x.w;
-    return r;
-}
 // The CTA's sums to *out.
 __device__ __forceinline__ void prs_block_sum(eg_red2 acc, float4 *s_sum, float4 *out) {
-    acc = prs_warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = make_float4(acc.s0, acc.c0, acc.s1, acc.c1);
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        acc = prs_warp_sum(prs_unpack(s_sum[threadIdx.x]));
-        if (threadIdx.x == 0) __stcg(out, make_float4(acc.s0, acc.c0, acc.s1, acc.c1));
-    }
+    acc = eg_block_sum(acc, s_sum);
+    if (threadIdx.x == 0) __stcg(out, acc.pack());
 }
 
 // REDUCE: the residual and the dangling mass are wanted (a tolerance, or
@@ -167,13 +142,13 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
 #pragma unroll
                     for (uint32_t k = 0; k < 8; k++) {
                         if (i0 + 32 * k >= G) break;
-                        const eg_red2 p = prs_unpack(x[k]);
+                        const eg_red2 p = eg_red2::unpack(x[k]);
                         sum.add(make_float2(p.s0, p.s1));
                         sum.c0 += p.c0;
                         sum.c1 += p.c1;
                     }
                 }
-                sum = prs_warp_sum(sum);
+                sum = eg_warp_sum(sum);
                 if (lane == 0) t = sum.wide();
             }
             if (lane == 0) {
