@@ -5,8 +5,7 @@
 // 191-197) and bfsgrid_cilk.c (get_bfs 48-65, iterator 121-168).  The
 // reference's frontier is a byte map plus id lists (random.c:74-77,
 // buffer.c:62-297); here it is a bitmap in the style of Gemini's Bitmap
-// (bitmap.h:16-50), written one 32-bit word per warp with __ballot_sync, plus
-// a compacted id queue for push levels.
+// (bitmap.h:16-50), plus a list with running edge sums for push levels.
 //
 // Levels follow the reference: level[root] = 1, unreached = 0 (the value
 // bfsgrid_cilk and the edge-centric bfs_simple write into dist[]).
@@ -14,18 +13,13 @@
 #include <string.h>
 
 #include "eg_bfsloop.cuh"
-#include "eg_bigwork.cuh"
 #include "eg_frontier.cuh"
 #include "eg_internal.cuh"
 #include "eg_mspull.cuh"
 
 namespace {
 
-// Frontier vertices of the multi-source push with more out-edges than this are
-// expanded by the whole grid (k_ms_push_big) instead of one warp, in chunks of
-// EG_BFS_CHUNK edges.
-#define EG_BFS_WARP_EDGES 256u
-#define EG_BFS_CHUNK 4096u
+#define EG_MS_STEP 4  // entries per lane in flight in the multi-source push
 
 // first[v] = v's in-neighbour with the largest out-degree (the smallest id
 // among equals), EG_NO_VERTEX when the in-list is empty: the in-neighbour
@@ -212,10 +206,10 @@ struct MsCounters {
     unsigned long long deg;   // sum of out-degrees of vertices with a nonzero new word
     unsigned long long tdeg;  // sum over new (vertex, source) pairs of the vertex's out-degree
     unsigned long long disc;  // new (vertex, source) pairs
+    unsigned long long sel;   // push: vertices listed by k_ms_queue << 32 | their entries
     uint32_t count;           // vertices with a nonzero new word
-    uint32_t nbig;            // frontier vertices deferred to k_ms_push_big; pull: k_msp_mid's list
+    uint32_t nheavy;          // pull: k_msp_mid's list
     uint32_t nhuge;           // pull: k_msp_heavy's list
-    uint32_t qlen;            // ids listed by k_ms_queue
 };
 
 __global__ void k_ms_init(uint32_t n, unsigned long long *seen, unsigned long long *front) {
@@ -289,112 +283,117 @@ __global__ void k_msg_prep(MsGState *st, MsCounters *cnt) {
     cnt->tdeg = 0;
     cnt->disc = 0;
     cnt->count = 0;
-    cnt->nbig = 0;
+    cnt->sel = 0;
+    cnt->nheavy = 0;
     cnt->nhuge = 0;
-    cnt->qlen = 0;
 }
 
-// Push levels: lists the vertices with a nonzero frontier word (four per
-// thread, one atomic per 1024 vertices).  The fold used to append them on
-// every level, one atomic per warp on the one counter.
+// Push levels: lists the vertices with a nonzero frontier word and out-edges
+// as (running sum of their entries, first entry - that sum, vertex); four
+// vertices per thread, one atomic per 1024 vertices.
 __global__ void __launch_bounds__(256) k_ms_queue(uint32_t n, const unsigned long long *__restrict__ front,
-                                                  uint32_t *queue, const MsGState *st, MsCounters *cnt) {
-    __shared__ uint32_t s_warp[8];
-    __shared__ uint32_t s_base;
+                                                  const uint32_t *__restrict__ ptr, uint4 *queue, const MsGState *st,
+                                                  MsCounters *cnt) {
+    __shared__ unsigned long long s_warp[8], s_base;
     if (st->pull) return;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint64_t b0 = blockIdx.x * 1024ull; b0 < n; b0 += gridDim.x * 1024ull) {
-        const uint64_t v0 = b0 + warp * 128u + lane;
-        uint32_t ball[4], c = 0;
+        const uint64_t v0 = b0 + 4 * threadIdx.x;
+        const uint32_t v = (uint32_t)v0;
+        uint32_t bits = 0, r[5];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (v0 + i < n && front[v0 + i] != 0ull) bits |= 1u << i;
+        bfsl_rows(ptr, v, bits != 0u, r);
+        unsigned long long mine = 0;  // vertices << 32 | entries (m < 2^32)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint64_t v = v0 + 32u * i;
-            ball[i] = __ballot_sync(EG_FULL_MASK, v < n && front[v] != 0ull);
-            c += __popc(ball[i]);
+            if (r[i + 1] == r[i]) bits &= ~(1u << i);
+            if ((bits >> i) & 1u) mine += (1ull << 32) | (r[i + 1] - r[i]);
         }
-        if (lane == 0) s_warp[warp] = c;
+        unsigned long long x = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(EG_FULL_MASK, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (lane == 31) s_warp[warp] = x;
         __syncthreads();
         if (threadIdx.x == 0) {
-            uint32_t t = 0;
+            unsigned long long t = 0;
             for (int w = 0; w < 8; w++) {
-                const uint32_t x = s_warp[w];
+                const unsigned long long y = s_warp[w];
                 s_warp[w] = t;
-                t += x;
+                t += y;
             }
-            s_base = t ? atomicAdd(&cnt->qlen, t) : 0u;
+            s_base = t ? atomicAdd(&cnt->sel, t) : 0ull;
         }
         __syncthreads();
-        uint32_t pos = s_base + s_warp[warp];
+        const unsigned long long at = s_base + s_warp[warp] + x - mine;
+        uint32_t pos = (uint32_t)(at >> 32), off = (uint32_t)at;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            if ((ball[i] >> lane) & 1u) queue[pos + __popc(ball[i] & eg_lanemask_lt())] = (uint32_t)(v0 + 32u * i);
-            pos += __popc(ball[i]);
+            if (!((bits >> i) & 1u)) continue;
+            queue[pos++] = make_uint4(off, r[i] - off, v + i, 0u);
+            off += r[i + 1] - r[i];
         }
         __syncthreads();  // s_warp and s_base are rewritten for the next 1024
     }
 }
 
-// Pull: a vertex ORs the frontier words of its in-neighbours, stopping early
-// once every source it still lacks has been found.
-// Push: 32 vertices with a nonzero frontier word per warp (eg_warp_lists); lists with more
-// than EG_BFS_WARP_EDGES out-edges go to a side list for k_ms_push_big.
-__global__ void __launch_bounds__(256) k_ms_push(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
-                                                 const uint32_t *__restrict__ queue, const MsGState *st,
-                                                 const unsigned long long *__restrict__ seen,
+// Push: every warp takes an equal share of the listed vertices' entries, hubs
+// included (eg_frontier.cuh's list), and hands each entry's vertex the sources
+// that it lacks.  Words read through L1 may be old: the atomicOr settles it.
+// Bound by its chain of loads and the launches around it.  (A warp walked 32
+// vertices' lists, the ones over 256 entries by chunks in two launches more:
+// list and push took 101 us of a 64-source batch on undirected RMAT n = 2^20,
+// now 41; of a 32-source one on n = 1.7K, m = 45K 88, now 29.)
+__global__ void __launch_bounds__(256) k_ms_push(const uint32_t *__restrict__ col, const uint4 *__restrict__ queue,
+                                                 const MsGState *st, const unsigned long long *__restrict__ seen,
                                                  const unsigned long long *__restrict__ front,
-                                                 unsigned long long *__restrict__ next, uint32_t *big,
-                                                 MsCounters *cnt) {
+                                                 unsigned long long *next, const MsCounters *cnt) {
     if (st->pull) return;
-    const uint32_t qlen = st->count;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    // 32 frontier vertices per warp, their lists walked together (eg_warp_lists)
-    for (uint32_t q0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; q0 < qlen; q0 += warps * 32) {
-        const uint32_t qi = q0 + lane;
-        uint32_t u = 0, b = 0, d = 0;
+    const uint32_t qlen = (uint32_t)(cnt->sel >> 32), E = (uint32_t)cnt->sel;
+    const uint32_t lane = threadIdx.x & 31, le = eg_lanemask_lt() | (1u << lane);
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t per = (uint32_t)(((uint64_t)E + warps - 1) / warps);
+    per = per < 64u ? 64u : (per + 31u) & ~31u;
+    const uint64_t begin = (uint64_t)wid * per;
+    if (begin >= E) return;
+    uint32_t p = (uint32_t)begin;
+    const uint32_t end = E - p > per ? p + per : E;
+    uint32_t i0 = eg_list_find(&queue[0].x, 4u, qlen, p);
+    for (; p < end; i0 += 32) {
+        uint4 q = make_uint4(0xffffffffu, 0u, 0u, 0u);
         unsigned long long f = 0ull;
-        if (qi < qlen) {
-            u = queue[qi];
-            b = ptr[u];
-            d = ptr[u + 1] - b;
-            if (d > EG_BFS_WARP_EDGES) {
-                big[atomicAdd(&cnt->nbig, 1u)] = u;
-                d = 0;
-            } else {
-                f = front[u];
-            }
+        if (i0 + lane < qlen) {
+            q = __ldg(queue + i0 + lane);
+            f = __ldg(front + q.z);
         }
-        eg_warp_lists(u, b, d, [&](bool valid, uint32_t lo, uint32_t, uint32_t p) {
-            const unsigned long long of = __shfl_sync(EG_FULL_MASK, f, lo);
-            if (valid) {
-                const uint32_t v = col[p];
-                const unsigned long long add = of & ~__ldcg(seen + v);
-                if (add && (__ldcg(next + v) & add) != add) atomicOr(next + v, add);
+        const uint32_t wend = i0 + 32 < qlen ? __ldg(&queue[i0 + 32].x) : E;
+        const uint32_t stop = wend < end ? wend : end;
+        for (; p < stop; p = stop - p > 32 * EG_MS_STEP ? p + 32 * EG_MS_STEP : stop) {
+            uint32_t v[EG_MS_STEP];
+            unsigned long long add[EG_MS_STEP], was[EG_MS_STEP];
+            bool on[EG_MS_STEP];
+#pragma unroll
+            for (int k = 0; k < EG_MS_STEP; k++) {
+                const uint32_t x0 = p + 32 * k;
+                const uint32_t starts = __reduce_or_sync(EG_FULL_MASK, q.x - x0 < 32u ? 1u << (q.x - x0) : 0u);
+                const uint32_t o = __popc(__ballot_sync(EG_FULL_MASK, q.x < x0)) - 1 + __popc(starts & le);
+                const uint32_t at = x0 + lane + __shfl_sync(EG_FULL_MASK, q.y, o);
+                add[k] = __shfl_sync(EG_FULL_MASK, f, o);
+                on[k] = stop - p > 32u * k + lane;
+                v[k] = on[k] ? __ldg(col + at) : 0u;
             }
-        });
-    }
-}
-
-// The deferred high-degree frontier vertices: every thread of the grid
-// strides over each one's out-list in turn.
-__global__ void __launch_bounds__(256) k_ms_push_big(const uint32_t *__restrict__ ptr,
-                                                     const uint32_t *__restrict__ col, const uint32_t *big,
-                                                     const uint32_t *__restrict__ bigoff,
-                                                     const unsigned long long *__restrict__ seen,
-                                                     const unsigned long long *__restrict__ front,
-                                                     unsigned long long *__restrict__ next, const MsCounters *cnt) {
-    const uint32_t nbig = *(volatile const uint32_t *)&cnt->nbig;
-    if (!nbig) return;
-    const uint32_t total = bigoff[nbig];
-    for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
-        const uint32_t i = eg_big_item(bigoff, nbig, c);
-        const uint32_t u = big[i];
-        const unsigned long long f = front[u];
-        const uint32_t b = ptr[u] + (c - bigoff[i]) * EG_BFS_CHUNK, e = min(ptr[u + 1], b + EG_BFS_CHUNK);
-        for (uint32_t p = b + threadIdx.x; p < e; p += blockDim.x) {
-            const uint32_t v = col[p];
-            const unsigned long long add = f & ~__ldcg(seen + v);
-            if (add && (__ldcg(next + v) & add) != add) atomicOr(next + v, add);
+#pragma unroll
+            for (int k = 0; k < EG_MS_STEP; k++) {
+                was[k] = on[k] ? __ldca(next + v[k]) : ~0ull;
+                add[k] &= on[k] ? ~__ldg(seen + v[k]) : 0ull;
+            }
+#pragma unroll
+            for (int k = 0; k < EG_MS_STEP; k++)
+                if (add[k] & ~was[k]) atomicOr(next + v[k], add[k]);
         }
     }
 }
@@ -490,12 +489,12 @@ __global__ void __launch_bounds__(256) k_ms_fold(uint32_t n, unsigned long long 
 }  // namespace
 
 // The level loop of eg_bfs_multi as one CUDA graph: a while node whose body
-// is prep (direction), push (+ hubs in chunks) or the two-part pull, fold,
+// is prep (direction), the push (list, entries) or the three-part pull, fold,
 // and end (counters into the state, loop condition).  Valid while the
 // buffers and k it was captured with (key) stay the same.
 static int msbfs_graph_build(eg_graph *g, const void *const key[8], const eg_adj *in_adj,
                              unsigned long long all, unsigned long long *seen, unsigned long long *front,
-                             unsigned long long *next, uint32_t *queue, uint32_t *big, uint32_t *bigoff, int32_t *levels,
+                             unsigned long long *next, uint4 *queue, int32_t *levels,
                              MsGState *st, MsCounters *cnt) {
     eg_ctx *ctx = g->ctx;
     eg_bfs_graph &bg = g->msg;
@@ -521,19 +520,16 @@ static int msbfs_graph_build(eg_graph *g, const void *const key[8], const eg_adj
     const uint32_t blocks = (uint32_t)ctx->sm_count * 8;
     EG_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     k_msg_prep<<<1, 1, 0, ctx->stream>>>(st, cnt);
-    k_ms_queue<<<blocks, 256, 0, ctx->stream>>>(n, front, queue, st, cnt);
-    k_ms_push<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(g->csr.ptr), bp<uint32_t>(g->csr.col), queue, st, seen,
-                                               front, next, big, cnt);
-    k_big_offsets<<<1, 1024, 0, ctx->stream>>>(big, &cnt->nbig, 1u, bp<uint32_t>(g->csr.ptr), EG_BFS_CHUNK, bigoff);
-    k_ms_push_big<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(g->csr.ptr), bp<uint32_t>(g->csr.col), big, bigoff,
-                                                   seen, front, next, cnt);
-    // the pull's lists reuse the push side list and queue (idle in a pull level)
+    k_ms_queue<<<blocks, 256, 0, ctx->stream>>>(n, front, bp<uint32_t>(g->csr.ptr), queue, st, cnt);
+    k_ms_push<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(g->csr.col), queue, st, seen, front, next, cnt);
+    // the pull's lists share the push's (idle in a pull level)
+    uint32_t *heavy = reinterpret_cast<uint32_t *>(queue), *huge = heavy + n;
     k_msp_light<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), n, all, seen,
-                                                 front, next, big, &cnt->nbig, &st->pull);
+                                                 front, next, heavy, &cnt->nheavy, &st->pull);
     k_msp_mid<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), all, seen, front,
-                                               next, big, &cnt->nbig, queue, &cnt->nhuge, &st->pull);
+                                               next, heavy, &cnt->nheavy, huge, &cnt->nhuge, &st->pull);
     k_msp_heavy<<<blocks, 256, 0, ctx->stream>>>(bp<uint32_t>(in_adj->ptr), bp<uint32_t>(in_adj->col), all, seen, front,
-                                                 next, queue, &cnt->nhuge, &st->pull);
+                                                 next, huge, &cnt->nhuge, &st->pull);
     k_ms_fold<<<blocks, 256, 0, ctx->stream>>>(n, seen, front, next, levels, st, deg, cnt);
     k_msg_end<<<1, 1, 0, ctx->stream>>>(st, cnt, handle);
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &body);
@@ -559,18 +555,14 @@ extern "C" int eg_bfs_multi(eg_graph *g, const uint32_t *roots, int k, int32_t *
     eg_ctx *ctx = g->ctx;
     EG_CUDA(cudaSetDevice(ctx->device));
     const uint32_t n = g->n;
-    // work: seen | front | next (u64 each) | queue (u32) | big list (u32) | roots | counters | state |
-    //       big chunk offsets
-    const uint64_t bytes = 3ull * n * 8 + 2ull * n * 4 + 64 * 4 + 64 + 64 + ((uint64_t)n + 1) * 4;
-    EG_TRY(eg_buf_ensure(ctx, g->msbfs_work, bytes));
-    unsigned long long *seen = bp<unsigned long long>(g->msbfs_work);
+    // work: push list (uint4) | seen | front | next (u64 each) | roots | counters | state
+    EG_TRY(eg_buf_ensure(ctx, g->msbfs_work, 40ull * n + 64 * 4 + 64 + 64));
+    uint4 *queue = bp<uint4>(g->msbfs_work);
+    unsigned long long *seen = reinterpret_cast<unsigned long long *>(queue + n);
     unsigned long long *front = seen + n, *next = seen + 2ull * n;
-    uint32_t *queue = reinterpret_cast<uint32_t *>(seen + 3ull * n);
-    uint32_t *big = queue + n;
-    uint32_t *d_roots = big + n;
+    uint32_t *d_roots = reinterpret_cast<uint32_t *>(seen + 3ull * n);
     MsCounters *cnt = reinterpret_cast<MsCounters *>(d_roots + 64);
     MsGState *st = reinterpret_cast<MsGState *>(d_roots + 64 + 16);
-    uint32_t *bigoff = d_roots + 64 + 32;
     int32_t *levels = nullptr;
     if (levels_out) {
         EG_TRY(eg_buf_ensure(ctx, g->level, (uint64_t)k * n * 4));
@@ -583,7 +575,7 @@ extern "C" int eg_bfs_multi(eg_graph *g, const uint32_t *roots, int k, int32_t *
     bool same = g->msg.exec != nullptr;
     for (int i = 0; i < 8 && same; i++) same = g->msg.key[i] == key[i];
     if (!same)
-        EG_TRY(msbfs_graph_build(g, key, in_adj, all, seen, front, next, queue, big, bigoff, levels, st, cnt));
+        EG_TRY(msbfs_graph_build(g, key, in_adj, all, seen, front, next, queue, levels, st, cnt));
     EG_CUDA(cudaMemcpyAsync(d_roots, roots, (uint64_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
     EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     if (levels) EG_CUDA(cudaMemsetAsync(levels, 0, (uint64_t)k * n * 4, ctx->stream));
