@@ -143,11 +143,10 @@ def run_ours(args):
     t0 = time.perf_counter()
     g.build(eg.CSR | eg.CSC)
     build_ms = g.info().build_ms
-    g.tune()  # row schedule and BFS level-loop form for this graph (untimed setup)
+    g.tune()  # row schedule and BFS switch divisor for this graph (untimed setup)
     roots = g.sample_roots(W["roots"], W["root_seed"])
     stream = torch.cuda.ExternalStream(ctx.stream)
-    # the BFS level-loop form: the tuner's (default), or fixed (a profiler
-    # slows per-level host round trips, so its own tuning would differ)
+    # host_loop as the caller asked (one level loop serves every value)
     bfs_form = {"auto": None, "graph": False, "host": True}[args.bfs_form]
 
     # host outputs of the end-to-end step: page-locked, allocated once and
@@ -649,9 +648,8 @@ def cache_report(ctx, eg, scale=24, path=None):
 
 
 def bfs_report(ctx, eg, scale=24, roots=16):
-    """Single-source BFS (levels + parents) on the undirected RMAT graph: the
-    CUDA-graph level loop and the host-driven loop (the same kernels launched
-    level by level, which a profiler can capture one by one), plus WCC."""
+    """Single-source BFS (levels + parents) on the undirected RMAT graph with
+    both values of host_loop (one level loop serves both), plus WCC."""
     n = 1 << scale
     g = ctx.rmat(scale, 16 * n, 2, undirected=True).build(eg.CSR | eg.CSC)
     rs = g.sample_roots(roots, 3)
@@ -717,7 +715,7 @@ def main():
     ap.add_argument("--scale", type=int, default=0)
     ap.add_argument("--no-extras", action="store_true")
     ap.add_argument("--bfs-form", choices=["auto", "graph", "host"], default="auto",
-                    help="BFS level loop: the form eg_graph_tune keeps (auto), or a fixed one")
+                    help="host_loop of the BFS calls (one level loop serves all three)")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--e2e-batch", type=int, default=E2E_BATCH, help="roots per eg_bfs_batch call in the end-to-end step")
     ap.add_argument("--pr-only", action="store_true", help="only the PageRank pull report (profiling)")

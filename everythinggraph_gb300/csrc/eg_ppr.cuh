@@ -7,11 +7,9 @@
 // entries per item: a whole row has at most EG_PPR_PART - 1 (its length order
 // is then one 9-bit sort pass), longer rows are cut into parts of EG_PPR_PART
 #define EG_PPR_PART 512u
-#ifndef EG_PPR_MINB
 // resident CTAs per SM of k_ppr_rows (48 registers).  RMAT-20 undirected, 32
 // queries: 3 325 us a sweep, 4 275, 5 249
 #define EG_PPR_MINB 5
-#endif
 
 namespace {
 
