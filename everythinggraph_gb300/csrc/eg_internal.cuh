@@ -283,12 +283,12 @@ __host__ __device__ __forceinline__ uint64_t eg_edge_hash(uint64_t seed, uint32_
 }
 
 // Two running sums (e.g. a residual and a dangling mass) kept by one thread
-// as fp32 (sum, error) pairs (Knuth's TwoSum), summed over the block in the
-// same form and widened to FP64 once per block.  FP64 instructions issue at a
-// small fraction of the fp32 rate on this GPU: per-row FP64 adds, often in
-// divergent code, would dominate the kernels that carry them, and FP64 sums
-// per warp cost PageRank's row pass over 12M entries 3 of its 51 us, the L1
-// change of 4M ranks 7 of its 13.
+// as fp32 (sum, error) pairs (Knuth's TwoSum), then summed over warps, blocks
+// and blocks' partials as fp32 triples (eg_sum2) and widened to FP64 once per
+// total.  FP64 instructions issue at a small fraction of the fp32 rate on this
+// GPU: per-row FP64 adds, often in divergent code, would dominate the kernels
+// that carry them, and FP64 sums per warp cost PageRank's row pass over 12M
+// entries 3 of its 51 us, the L1 change of 4M ranks 7 of its 13.
 struct eg_red2 {
     float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f;
     __device__ __forceinline__ static void two_sum(float &s, float &c, float x) {
@@ -304,38 +304,114 @@ struct eg_red2 {
     __device__ __forceinline__ double2 wide() const {
         return make_double2((double)s0 + (double)c0, (double)s1 + (double)c1);
     }
-    __device__ __forceinline__ float4 pack() const { return make_float4(s0, c0, s1, c1); }
-    __device__ __forceinline__ static eg_red2 unpack(float4 x) {
-        eg_red2 r;
-        r.s0 = x.x;
-        r.c0 = x.y;
-        r.s1 = x.z;
-        r.c1 = x.w;
+};
+// A sum as three fp32 words of falling weight.  Adding two of them keeps the
+// first two words' rounding errors in the third, so that a tree of additions
+// is off by about 2^-70 of the total, less than FP64's 2^-53 per addition
+// (pairs alone: 2^-48).
+struct eg_sum3 {
+    float s = 0.f, c = 0.f, e = 0.f;
+    __device__ __forceinline__ static eg_sum3 of(double x) {  // the nearest triple (x itself, within fp32's range)
+        eg_sum3 r;
+        r.s = (float)x;
+        if (isinf(r.s)) return r;
+        r.c = (float)(x - (double)r.s);
+        r.e = (float)((x - (double)r.s) - (double)r.c);
         return r;
     }
+    __device__ __forceinline__ void add(const eg_sum3 &y) {
+        float err = 0.f;
+        e += y.e;
+        eg_red2::two_sum(s, err, y.s);
+        eg_red2::two_sum(c, e, y.c);
+        eg_red2::two_sum(c, e, err);
+    }
+    __device__ __forceinline__ void add(float x) {
+        float err = 0.f;
+        eg_red2::two_sum(s, err, x);
+        eg_red2::two_sum(c, e, err);
+    }
+    __device__ __forceinline__ double wide() const { return (double)s + ((double)c + (double)e); }
 };
-// A warp's sums in its lane 0.
-__device__ __forceinline__ eg_red2 eg_warp_sum(eg_red2 acc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float s0 = __shfl_down_sync(0xffffffffu, acc.s0, o), c0 = __shfl_down_sync(0xffffffffu, acc.c0, o);
-        const float s1 = __shfl_down_sync(0xffffffffu, acc.s1, o), c1 = __shfl_down_sync(0xffffffffu, acc.c1, o);
-        acc.add(make_float2(s0, s1));
-        acc.c0 += c0;
-        acc.c1 += c1;
+struct __align__(8) eg_sum2 {
+    eg_sum3 a, b;
+    eg_sum2() = default;
+    __device__ __forceinline__ explicit eg_sum2(const eg_red2 &r) {
+        a.s = r.s0;
+        a.c = r.c0;
+        b.s = r.s1;
+        b.c = r.c1;
     }
-    return acc;
+};
+__device__ __forceinline__ eg_sum3 eg_shfl_xor(const eg_sum3 &x, int o) {
+    eg_sum3 y;
+    y.s = __shfl_xor_sync(EG_FULL_MASK, x.s, o);
+    y.c = __shfl_xor_sync(EG_FULL_MASK, x.c, o);
+    y.e = __shfl_xor_sync(EG_FULL_MASK, x.e, o);
+    return y;
 }
-// The block's sums in thread 0 (whole warps; s_sum: 32 entries).
-__device__ __forceinline__ eg_red2 eg_block_sum(eg_red2 acc, float4 *s_sum) {
-    acc = eg_warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc.pack();
+// Half warps' sums, in all their lanes.
+__device__ __forceinline__ eg_sum3 eg_half_sum(eg_sum3 x) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) x.add(eg_shfl_xor(x, o));
+    return x;
+}
+// A warp's sums: a's in lanes 0 .. 15, b's in lanes 16 .. 31.  The halves trade
+// the sum that they do not keep first: one triple per lane and step, where two
+// cost k_pr_small 0.6 us an iteration.
+__device__ __forceinline__ eg_sum3 eg_warp_sum(const eg_sum2 &x) {
+    const bool hi = threadIdx.x & 16;
+    eg_sum3 mine = hi ? x.b : x.a;
+    mine.add(eg_shfl_xor(hi ? x.a : x.b, 16));
+    return eg_half_sum(mine);
+}
+// The block's sums in warp 0, placed the same, from its warps' (whole warps;
+// s_sum: 32 entries).
+__device__ __forceinline__ eg_sum3 eg_block_sum(eg_sum3 x, eg_sum2 *s_sum) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (!(lane & 15)) (lane ? s_sum[threadIdx.x >> 5].b : s_sum[threadIdx.x >> 5].a) = x;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        acc = threadIdx.x < (blockDim.x >> 5) ? eg_red2::unpack(s_sum[threadIdx.x]) : eg_red2();
-        acc = eg_warp_sum(acc);
+    if (threadIdx.x < 32) x = eg_warp_sum(lane < (blockDim.x >> 5) ? s_sum[lane] : eg_sum2());
+    return x;
+}
+__device__ __forceinline__ eg_sum3 eg_block_sum(const eg_sum2 &acc, eg_sum2 *s_sum) {
+    return eg_block_sum(eg_warp_sum(acc), s_sum);
+}
+// A block's sums (as eg_block_sum leaves them) to *out.
+__device__ __forceinline__ void eg_store_sum(const eg_sum3 &x, eg_sum2 *out) {
+    if (threadIdx.x >= 32 || (threadIdx.x & 15)) return;
+    float *p = reinterpret_cast<float *>(out) + (threadIdx.x ? 3 : 0);
+    __stcg(p, x.s);
+    __stcg(p + 1, x.c);
+    __stcg(p + 2, x.e);
+}
+// A half warp's word of a partial (lanes 0 .. 15: a, 16 .. 31: b), not through
+// L1: other SMs write them.
+__device__ __forceinline__ eg_sum3 eg_load_sum(const eg_sum2 *part, bool on) {
+    const float *p = reinterpret_cast<const float *>(part) + (threadIdx.x & 16 ? 3 : 0);
+    eg_sum3 x;
+    if (on) {
+        x.s = __ldcg(p);
+        x.c = __ldcg(p + 1);
+        x.e = __ldcg(p + 2);
     }
-    return acc;
+    return x;
+}
+// The total of blocks' partials (the first warp's lane 0), from its triples:
+// widened, or, where a total leaves fp32's range, the FP64 sum of the partials.
+__device__ __forceinline__ double2 eg_total(const eg_sum3 &sum, const eg_sum2 *part, uint32_t nparts) {
+    double t = 0.0;
+    if (__all_sync(EG_FULL_MASK, isfinite(sum.s))) {
+        t = sum.wide();
+    } else {
+        for (uint32_t i = 0; i < nparts; i += 16) {
+            const uint32_t k = i + (threadIdx.x & 15);
+            t += eg_load_sum(part + k, k < nparts).wide();
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(EG_FULL_MASK, t, o);
+    }
+    return make_double2(t, __shfl_down_sync(EG_FULL_MASK, t, 16));
 }
 
 // SSSP edge weights computed from the endpoints (no weight array), and the

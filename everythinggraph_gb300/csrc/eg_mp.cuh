@@ -21,7 +21,8 @@
 //   float2 emit(row, A)       finishes a row; the two partials it returns
 //                             (PageRank: |change|, dangling mass) are summed
 //                             per thread as fp32 TwoSum pairs (eg_red2), then
-//                             per CTA in FP64, when REDUCE is set
+//                             per CTA as fp32 triples (eg_sum2; the merge-path
+//                             kernels: in FP64), when REDUCE is set
 #pragma once
 #include <type_traits>
 #include "eg_internal.cuh"
@@ -320,10 +321,9 @@ struct eg_f2sum {
 
 // The block's share of the emitted (residual, dangling) partials into part[blockIdx.x].
 template <bool REDUCE>
-__device__ __forceinline__ void eg_block_part(const eg_red2 &redf, float4 *__restrict__ part, float4 *s_red) {
+__device__ __forceinline__ void eg_block_part(const eg_red2 &redf, eg_sum2 *__restrict__ part, eg_sum2 *s_red) {
     if (!REDUCE) return;
-    const eg_red2 sum = eg_block_sum(redf, s_red);
-    if (threadIdx.x == 0) part[blockIdx.x] = sum.pack();
+    eg_store_sum(eg_block_sum(eg_sum2(redf), s_red), part + blockIdx.x);
 }
 
 // Rows split between warp tiles, finished from the tiles' head and tail
@@ -429,8 +429,8 @@ __device__ __forceinline__ void eg_coo_empty_range(uint32_t b, uint32_t nb, uint
 template <class Op, int TILE_E, bool REDUCE, int EMPTY>
 __global__ void k_coo_tail(const uint32_t *__restrict__ ptr, uint32_t n, uint32_t empty_from, uint32_t ntiles,
                            uint32_t gf, const eg_mp_carry<typename Op::A> *__restrict__ carry,
-                           float4 *__restrict__ part, Op op) {
-    __shared__ float4 s_red[32];
+                           eg_sum2 *__restrict__ part, Op op) {
+    __shared__ eg_sum2 s_red[32];
     if (!op.active()) return;
     op.setup();
     eg_red2 redf;
@@ -449,8 +449,8 @@ __global__ void k_coo_tail(const uint32_t *__restrict__ ptr, uint32_t n, uint32_
 
 // The range alone (layouts whose row kernel splits no rows).
 template <class Op, bool REDUCE>
-__global__ void k_coo_empty_range(uint32_t lo, uint32_t hi, float4 *__restrict__ part, Op op) {
-    __shared__ float4 s_red[32];
+__global__ void k_coo_empty_range(uint32_t lo, uint32_t hi, eg_sum2 *__restrict__ part, Op op) {
+    __shared__ eg_sum2 s_red[32];
     if (!op.active()) return;
     op.setup();
     eg_red2 redf;
@@ -766,13 +766,13 @@ template <class Op, int TILE_E, int U, bool REDUCE, int PF = 0, int MINB = 6, in
 __global__ void __launch_bounds__(256, MINB) k_coov_rows(const uint32_t *__restrict__ rid,
                                                          const uint32_t *__restrict__ col, uint32_t m, uint32_t ntiles,
                                                          eg_mp_carry<typename Op::A> *__restrict__ carry,
-                                                         float4 *__restrict__ part, Op op,
+                                                         eg_sum2 *__restrict__ part, Op op,
                                                          const uint32_t *__restrict__ starts = nullptr,
                                                          const uint32_t *__restrict__ trow = nullptr) {
     static_assert(U == 4 || U == 8, "4 or 8 entries per lane");
     static_assert(TILE_E % (32 * U) == 0, "tiles hold whole chunks");
     static_assert(!MK || TILE_E % EG_TROW_SPAN == 0, "tiles start at a row sample");
-    __shared__ float4 s_red[32];
+    __shared__ eg_sum2 s_red[32];
     if (!op.active()) return;
     op.setup();
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(EG_PC_THREADS, EG_PC_CTAS)
     k_pcol_rows(const uint4 *__restrict__ seg, uint32_t nseg, const uint32_t *__restrict__ dst,
                 const uint32_t *__restrict__ ridx, const uint32_t *__restrict__ crun,
                 const uint32_t *__restrict__ rsrc, unsigned long long *__restrict__ gacc,
-                uint32_t *__restrict__ ticket, uint32_t parts, uint32_t rows, float4 *__restrict__ part, Op op,
+                uint32_t *__restrict__ ticket, uint32_t parts, uint32_t rows, eg_sum2 *__restrict__ part, Op op,
                 float fx, float fx_inv) {
     using T = unsigned long long;
     constexpr uint32_t D = 1u << SHIFT;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(EG_PC_THREADS, EG_PC_CTAS)
     uint32_t *slo = reinterpret_cast<uint32_t *>(eg_pc_sm);                    // low words
     uint32_t *shi = reinterpret_cast<uint32_t *>(eg_pc_sm + SM::word_bytes);  // high words
     auto row_sum = [&](uint32_t l) -> float { return eg_u642f_rn(shi[l], slo[l]) * fx_inv; };
-    __shared__ float4 s_red[32];
+    __shared__ eg_sum2 s_red[32];
     __shared__ uint32_t s_seg;
     __shared__ int s_last;
     if (!op.active()) return;

@@ -213,21 +213,16 @@ __global__ void __launch_bounds__(256) k_ppr_finish(const float *__restrict__ Y,
             X4[at] = make_float4(x[0], x[1], x[2], x[3]);
         }
     }
-    // the four groups' pairs are merged in fp32 pairs, then widened
+    // the four groups' pairs are merged as fp32 triples, then widened
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-#pragma unroll
-        for (int o = 8; o < 32; o <<= 1) {
-            eg_red2 y;
-            y.s0 = __shfl_xor_sync(EG_FULL_MASK, acc[j].s0, o);
-            y.c0 = __shfl_xor_sync(EG_FULL_MASK, acc[j].c0, o);
-            y.s1 = __shfl_xor_sync(EG_FULL_MASK, acc[j].s1, o);
-            y.c1 = __shfl_xor_sync(EG_FULL_MASK, acc[j].c1, o);
-            acc[j].add(make_float2(y.s0, y.s1));
-            acc[j].c0 += y.c0;
-            acc[j].c1 += y.c1;
-        }
-        if (grp == 0) s_part[warp][4 * sl + j] = acc[j].wide();
+        const eg_sum2 sum(acc[j]);  // groups 0 and 1 keep the first sum, 2 and 3 the second
+        eg_sum3 mine = grp < 2 ? sum.a : sum.b;
+        mine.add(eg_shfl_xor(grp < 2 ? sum.b : sum.a, 16));
+        mine.add(eg_shfl_xor(mine, 8));
+        const double w = mine.wide();
+        if (grp == 0) s_part[warp][4 * sl + j].x = w;
+        if (grp == 2) s_part[warp][4 * sl + j].y = w;
     }
     __syncthreads();
     if (warp == 0) {

@@ -146,42 +146,48 @@ struct PrAccOp {
 
 // rank = prev_init, contrib = prev_init / deg; partial dangling mass
 __global__ void k_pr_init(uint32_t n, float prev_init, const uint32_t *__restrict__ deg, uint32_t mult,
-                          float *__restrict__ rank, float *__restrict__ contrib, float4 *__restrict__ part) {
-    __shared__ float4 s_red[32];
-    eg_red2 dang;
+                          float *__restrict__ rank, float *__restrict__ contrib, eg_sum2 *__restrict__ part) {
+    __shared__ uint32_t s_none[8];
+    uint32_t none = 0;  // vertices without out-edges
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         uint32_t d = deg[v] * mult;
         rank[v] = prev_init;
         contrib[v] = d ? __fdiv_rn(prev_init, (float)d) : 0.f;
-        if (!d) dang.add(make_float2(0.f, prev_init));
+        none += !d;
     }
-    dang = eg_block_sum(dang, s_red);
-    if (threadIdx.x == 0) part[blockIdx.x] = dang.pack();
+    none = __reduce_add_sync(EG_FULL_MASK, none);
+    if ((threadIdx.x & 31) == 0) s_none[threadIdx.x >> 5] = none;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) none += s_none[w];
+        eg_sum2 p;
+        p.b = eg_sum3::of((double)none * (double)prev_init);
+        part[blockIdx.x] = p;
+    }
 }
 
 // Personalised start vector: multiplicity / total seeds on the seeds, 0 elsewhere.
 __global__ void k_ppr1_init(uint32_t n, PprSeeds seeds, float inv_total, const uint32_t *__restrict__ deg,
-                            float *__restrict__ rank, float *__restrict__ contrib, float4 *__restrict__ part) {
-    __shared__ float4 s_red[32];
-    eg_red2 dang;
+                            float *__restrict__ rank, float *__restrict__ contrib, eg_sum2 *__restrict__ part) {
+    __shared__ eg_sum2 s_red[32];
+    eg_sum2 dang;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const uint32_t d = deg[v];
         const float r = seeds.weight(v) * inv_total;
         rank[v] = r;
         contrib[v] = d ? __fdiv_rn(r, (float)d) : 0.f;
-        if (!d) dang.add(make_float2(0.f, r));
+        if (!d) dang.b.add(r);
     }
-    dang = eg_block_sum(dang, s_red);
-    if (threadIdx.x == 0) part[blockIdx.x] = dang.pack();
+    eg_store_sum(eg_block_sum(dang, s_red), part + blockIdx.x);
 }
 
 // L1 change between two rank vectors, per-block partials in the first sum (the
 // stop test's residual); skipped once the run has converged.
 __global__ void k_pr_residual(const float *__restrict__ cur, const float *__restrict__ prev, uint32_t n,
-                              const eg_pr_dev *st, float4 *__restrict__ part) {
-    __shared__ float4 s_red[32];
+                              const eg_pr_dev *st, eg_sum2 *__restrict__ part) {
+    __shared__ eg_sum2 s_red[32];
     if (st->done) return;
-    eg_red2 acc;
+    eg_sum2 acc;
     const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);  // 16 bytes per load (the arrays' ends are padded)
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const float4 c = __ldg(reinterpret_cast<const float4 *>(cur) + q);
@@ -190,10 +196,9 @@ __global__ void k_pr_residual(const float *__restrict__ cur, const float *__rest
         const float d[4] = {fabsf(c.x - p.x), left > 1 ? fabsf(c.y - p.y) : 0.f, left > 2 ? fabsf(c.z - p.z) : 0.f,
                             left > 3 ? fabsf(c.w - p.w) : 0.f};
 #pragma unroll
-        for (int k = 0; k < 4; k++) eg_red2::two_sum(acc.s0, acc.c0, d[k]);
+        for (int k = 0; k < 4; k++) acc.a.add(d[k]);
     }
-    acc = eg_block_sum(acc, s_red);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc.pack();
+    eg_store_sum(eg_block_sum(acc, s_red), part + blockIdx.x);
 }
 
 __global__ void k_map_ids(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ in, uint32_t k,
@@ -211,25 +216,23 @@ __global__ void k_pr_unpermute(const float *__restrict__ rank_a, const float *__
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) rank[v] = src[perm[v]];
 }
 
-// One block: deterministic sum of the partials, widened to FP64 at the end;
-// next base, stop test.  fp32 pairs: 7.0 us for 6.2K partials and 2.1 for none,
-// 15.4 and 3.2 as FP64 sums.
+// One block: deterministic sum of the partials' triples, widened to FP64 at the
+// end; next base, stop test.  (As FP64 sums 15.4 us for 6.2K partials, 3.2 for
+// none.)
 #define EG_PR_RED_T 512
-__global__ void k_pr_reduce(const float4 *__restrict__ part, uint32_t nparts, eg_pr_dev *st, double tele_div,
+__global__ void k_pr_reduce(const eg_sum2 *__restrict__ part, uint32_t nparts, eg_pr_dev *st, double tele_div,
                             float damping, int dangling, double tol, int count_iter) {
-    __shared__ float4 s[32];
+    __shared__ eg_sum2 s[32];
     if (st->done) return;
-    eg_red2 acc;
+    eg_sum3 acc;  // half warps take one of the two sums each
 #pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < nparts; i += EG_PR_RED_T) {
-        const float4 p = part[i];
-        acc.add(make_float2(p.x, p.z));
-        acc.c0 += p.y;
-        acc.c1 += p.w;
-    }
-    if (nparts) acc = eg_block_sum(acc, s);
+    for (uint32_t i = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15); i < nparts; i += EG_PR_RED_T / 2)
+        acc.add(eg_load_sum(part + i, true));
+    if (nparts) acc = eg_block_sum(eg_half_sum(acc), s);
+    if (threadIdx.x >= 32) return;
+    const double2 total = eg_total(acc, part, nparts);
     if (threadIdx.x == 0) {
-        const double res = acc.wide().x, dang = acc.wide().y;
+        const double res = total.x, dang = total.y;
         st->residual = res;
         st->dangling = dang;
         double b = (1.0 - (double)damping) / tele_div;
@@ -284,7 +287,7 @@ template <class Op>
 struct coo_spmv : std::false_type {};
 
 template <class Op, int TILE, int U, bool REDUCE, int PF, int MINB, int HINT = 0, bool MK = false>
-static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *part, const Op &op, uint32_t *nparts,
+static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, eg_sum2 *part, const Op &op, uint32_t *nparts,
                         cudaEvent_t ev_begin, cudaEvent_t ev_end, uint64_t m_entries, bool empty_rows,
                         uint32_t empty_from) {
     static_assert(!MK || TILE % EG_TROW_SPAN == 0, "masked tiles start at a row sample");
@@ -313,7 +316,7 @@ static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *par
     }
     if (g2 + gf) {
         const auto *carry = bp<eg_mp_carry<A>>(carry_buf);
-        float4 *tail = part ? part + g1_parts : nullptr;
+        eg_sum2 *tail = part ? part + g1_parts : nullptr;
         const uint32_t *ptr = bp<uint32_t>(adj.ptr);
         if constexpr (MK) {
             if (!ranged) return eg_fail(EG_EINVAL, "masked rows without an empty range");
@@ -335,7 +338,7 @@ static int coo_launch_t(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *par
 // empty_from <= n: the rows without entries are exactly [empty_from, n).
 // MK: `adj` is the relabelled CSC, read through its row-start bits.
 template <class Op, bool REDUCE, bool MK = false>
-static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *part, const Op &op, uint32_t *nparts,
+static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, eg_sum2 *part, const Op &op, uint32_t *nparts,
                       cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr,
                       uint64_t m_entries = EG_ALL_ENTRIES, bool empty_rows = true, uint32_t empty_from = EG_NO_RANGE) {
 #define EG_ROW_CASE(i, T, U, PF, MB, H)                                                                             \
@@ -392,7 +395,7 @@ static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, float4 *part,
 #endif
 #define EG_PR_CANDS (EG_ROW_CFGS + 1)  // the tuner's candidates: the row schedules, then the partition kernel
 template <bool REDUCE>
-static int pcol_launch(eg_graph *g, const PrOp<false> &op, float4 *part, uint32_t *nparts, cudaEvent_t ev_begin,
+static int pcol_launch(eg_graph *g, const PrOp<false> &op, eg_sum2 *part, uint32_t *nparts, cudaEvent_t ev_begin,
                        cudaEvent_t ev_end, bool empty_rows, double mass) {
     eg_ctx *ctx = g->ctx;
     eg_pcols &pc = g->pcol;
@@ -482,7 +485,7 @@ static uint32_t pr_block_log2(const eg_graph *g, const eg_pr_opts &o) {
 // EG_KEV iterations are bracketed by the context's kernel events.
 template <bool COMP, bool REDUCE>
 static int pr_iterations(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, double tele_div, eg_pr_dev *st,
-                         float4 *part, eg_buf &carry, bool timed, int it0, int it1) {
+                         eg_sum2 *part, eg_buf &carry, bool timed, int it0, int it1) {
     eg_ctx *ctx = g->ctx;
     for (int it = it0; it < it1; it++) {
         PrOp<COMP> op;
@@ -564,7 +567,7 @@ static int pr_iterations(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, d
 
 // Iterations [it0, it1).
 static int pr_dispatch(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, double tele_div, bool reduce,
-                       eg_pr_dev *st, float4 *part, eg_buf &carry, bool timed, int it0, int it1) {
+                       eg_pr_dev *st, eg_sum2 *part, eg_buf &carry, bool timed, int it0, int it1) {
     if (o.compensated) {
         if (reduce) return pr_iterations<true, true>(g, o, ps, tele_div, st, part, carry, timed, it0, it1);
         return pr_iterations<true, false>(g, o, ps, tele_div, st, part, carry, timed, it0, it1);
@@ -575,7 +578,7 @@ static int pr_dispatch(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, dou
 
 // The iteration loop of plain PageRank captured once as a CUDA graph and
 // replayed while the options and the buffers it was captured with stay the same.
-static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st, float4 *part, eg_buf &carry) {
+static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st, eg_sum2 *part, eg_buf &carry) {
     eg_ctx *ctx = g->ctx;
     uint64_t key[16] = {};
     key[0] = (uint32_t)o.iterations | ((uint64_t)g->csc_p_rows << 32);
@@ -641,7 +644,7 @@ static int pr_run_small(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr
     const uint32_t n = g->n, m = (uint32_t)g->m;
     const uint32_t want = eg_div_up(m, EG_PRS_SHARE), G = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
     for (eg_buf *b : {&g->rank, &g->rank_p, &g->contrib0, &g->contrib1}) EG_TRY(eg_buf_ensure(ctx, *b, (uint64_t)n * 4));
-    EG_TRY(eg_buf_ensure(ctx, g->pr_part, 2ull * G * sizeof(float4)));
+    EG_TRY(eg_buf_ensure(ctx, g->pr_part, 2ull * G * sizeof(eg_sum2)));
     eg_pr_dev *st = bp<eg_pr_dev>(g->pr_stats);
     const bool reduce = o.tolerance > 0.0 || o.dangling;
     const bool stage = n <= EG_PRS_STAGE_N;
@@ -652,7 +655,7 @@ static int pr_run_small(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr
               n, g->csc_p_rows, m, o.deg_multiplier, o.iterations, o.swap, o.dangling, o.damping,
               o.prev_init < 0.f ? 1.0f / (float)n : o.prev_init, (1.0 - (double)o.damping) / (double)n,
               (double)o.damping / (double)n, o.tolerance, bp<float>(g->contrib0), bp<float>(g->contrib1),
-              bp<float>(g->rank_p), bp<float>(g->rank), bp<float4>(g->pr_part), st,
+              bp<float>(g->rank_p), bp<float>(g->rank), bp<eg_sum2>(g->pr_part), st,
               (uint32_t)(share < cap ? share : cap)};
     const size_t smem = (size_t)(fixed + ((a.cap * cw + 15) & ~15ull));
     const void *fn = stage ? (reduce ? (const void *)k_pr_small<true, true> : (const void *)k_pr_small<false, true>)
@@ -689,12 +692,12 @@ static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t
     EG_TRY(eg_buf_ensure(ctx, g->rank_q, (uint64_t)n * 4));
     EG_TRY(eg_buf_ensure(ctx, g->contrib0, (uint64_t)n * 4));
     EG_TRY(eg_buf_ensure(ctx, g->contrib1, (uint64_t)n * 4));
-    EG_TRY(eg_buf_ensure(ctx, g->pr_part, ((uint64_t)nparts + 1024) * sizeof(float4)));
+    EG_TRY(eg_buf_ensure(ctx, g->pr_part, ((uint64_t)nparts + 1024) * sizeof(eg_sum2)));
     eg_buf &carry = g->mp_carry;
     eg_pr_dev *st = bp<eg_pr_dev>(g->pr_stats);
-    float4 *part = bp<float4>(g->pr_part);
+    eg_sum2 *part = bp<eg_sum2>(g->pr_part);
     EG_CUDA(cudaMemsetAsync(st, 0, sizeof(eg_pr_dev), ctx->stream));
-    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(float4), ctx->stream));
+    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(eg_sum2), ctx->stream));
     const bool ppr = ps.count > 0;
     const double tele_div = ppr ? (double)seed_total : (double)n;
     const bool reduce = o.tolerance > 0.0 || o.dangling;
@@ -711,7 +714,7 @@ static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t
     EG_LAUNCHED(ctx);
     k_pr_reduce<<<1, EG_PR_RED_T, 0, ctx->stream>>>(part, ib, st, tele_div, o.damping, o.dangling, 0.0, 0);
     EG_LAUNCHED(ctx);
-    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(float4), ctx->stream));
+    EG_CUDA(cudaMemsetAsync(part, 0, ((uint64_t)nparts + 1024) * sizeof(eg_sum2), ctx->stream));
     const bool graph = o.use_graph && !ppr;
     if (graph) EG_TRY(pr_graph(g, o, reduce, st, part, carry));
     EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));

@@ -11,7 +11,7 @@
 // gathered from L2 (L1 could hold the last iteration's).  A row is summed by one lane up to EG_PRS_LANE
 // entries, by 8 lanes up to EG_PRS_GROUP, by a warp up to EG_PRS_WARP, else by
 // the CTA; the order is fixed, so a run's bits are too.  The residual and the
-// dangling mass are summed as fp32 TwoSum pairs to the end and widened once:
+// dangling mass are summed as fp32 triples and widened once:
 // FP64 issues so slowly here that an FP64 pair per warp was half an iteration.
 //
 // Ten iterations (or to 1e-6), one call, before -> now: 1,250 vertices 354 ->
@@ -48,7 +48,7 @@ struct PrSmall {
     float damping, prev_init;
     double base0, per_dangling, tol;  // base = base0 + per_dangling * dangling mass
     float *c0, *c1, *rank_p, *rank;
-    float4 *part;  // two sets of one TwoSum pair of sums per CTA
+    eg_sum2 *part;  // two sets of one pair of sums per CTA
     eg_pr_dev *st;
     uint32_t cap;  // columns kept in shared memory
 };
@@ -70,18 +70,12 @@ __device__ __forceinline__ uint32_t prs_rows_below(const uint32_t *__restrict__ 
     return lo;
 }
 
-// The CTA's sums to *out.
-__device__ __forceinline__ void prs_block_sum(eg_red2 acc, float4 *s_sum, float4 *out) {
-    acc = eg_block_sum(acc, s_sum);
-    if (threadIdx.x == 0) __stcg(out, acc.pack());
-}
-
 // REDUCE: the residual and the dangling mass are wanted (a tolerance, or
 // dangling mass spread).
 template <bool REDUCE, bool STAGE>
 __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a) {
     extern __shared__ __align__(16) unsigned char prs_raw[];
-    __shared__ float4 s_sum[EG_PRS_THREADS / 32];
+    __shared__ eg_sum2 s_sum[EG_PRS_THREADS / 32];
     __shared__ float s_part[EG_PRS_THREADS / 32];
     __shared__ uint32_t s_row[2], s_long[EG_PRS_MAX_LONG], s_nlong;
     __shared__ float s_base;
@@ -105,12 +99,12 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
         if (__ldg(a.ptr + r + 1) - __ldg(a.ptr + r) > EG_PRS_WARP) s_long[atomicAdd(&s_nlong, 1u)] = r;
     // the start vector, in equal shares of the vertices
     const uint32_t per = (a.n + G - 1) / G, v0 = b * per < a.n ? b * per : a.n, v1 = a.n - v0 < per ? a.n : v0 + per;
-    eg_red2 acc;
+    eg_sum2 acc;
     for (uint32_t v = v0 + tid; v < v1; v += EG_PRS_THREADS) {
         const uint32_t d = __ldg(a.deg + v) * a.mult;
         __stcg(a.rank_p + v, a.prev_init);
         __stcg(a.c0 + v, d ? __fdiv_rn(a.prev_init, (float)d) : 0.f);
-        acc.add(make_float2(0.f, d ? 0.f : a.prev_init));
+        acc.b.add(d ? 0.f : a.prev_init);
     }
     __syncthreads();
     if (tid == 0)  // in row order, so that the sums below keep one order
@@ -120,7 +114,7 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
                 s_long[j] = s_long[j - 1];
                 s_long[j - 1] = t;
             }
-    if (REDUCE) prs_block_sum(acc, s_sum, a.part + b);
+    if (REDUCE) eg_store_sum(eg_block_sum(acc, s_sum), a.part + b);
     const uint32_t eper = (a.n - a.rows + G - 1) / G;  // rows without entries, in equal shares
     const uint32_t x0 = a.n - a.rows > b * eper ? a.rows + b * eper : a.n, x1 = a.n - x0 < eper ? a.n : x0 + eper;
     for (int it = 0;; it++) {
@@ -132,24 +126,16 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
         if (warp == 0) {
             double2 t = make_double2(0.0, 0.0);
             if (REDUCE) {
-                const float4 *part = a.part + (it & 1) * G;
-                eg_red2 sum;
-                for (uint32_t i0 = 0; i0 < G; i0 += 256) {  // all of a lane's loads in flight
-                    float4 x[8];
+                const eg_sum2 *part = a.part + (it & 1) * G;
+                eg_sum3 sum;
+                for (uint32_t i0 = lane & 15; i0 < G; i0 += 80) {  // five of a lane's loads in flight
+                    eg_sum3 x[5];
 #pragma unroll
-                    for (uint32_t k = 0; k < 8; k++)
-                        x[k] = i0 + 32 * k + lane < G ? __ldcg(part + i0 + 32 * k + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (uint32_t k = 0; k < 5; k++) x[k] = eg_load_sum(part + i0 + 16 * k, i0 + 16 * k < G);
 #pragma unroll
-                    for (uint32_t k = 0; k < 8; k++) {
-                        if (i0 + 32 * k >= G) break;
-                        const eg_red2 p = eg_red2::unpack(x[k]);
-                        sum.add(make_float2(p.s0, p.s1));
-                        sum.c0 += p.c0;
-                        sum.c1 += p.c1;
-                    }
+                    for (uint32_t k = 0; k < 5; k++) sum.add(x[k]);
                 }
-                sum = eg_warp_sum(sum);
-                if (lane == 0) t = sum.wide();
+                t = eg_total(eg_half_sum(sum), part, G);
             }
             if (lane == 0) {
                 s_base = (float)(a.dangling ? a.base0 + a.per_dangling * t.y : a.base0);
@@ -171,7 +157,7 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
         __syncthreads();
         if (s_done) break;
         const float base = s_base;
-        acc = eg_red2();
+        acc = eg_sum2();
         auto gather = [&](uint32_t e) -> float {
             const uint32_t i = e - E0;
             const uint32_t u = i < kept ? (uint32_t)s_col[i] : __ldg(a.col + e);
@@ -182,7 +168,10 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
         auto emit = [&](uint32_t r, float s, float old) {
             const float x = fmaf(a.damping, s, base);
             const uint32_t d = __ldg(a.deg + r) * a.mult;
-            if (REDUCE) acc.add(make_float2(fabsf(x - old), d ? 0.f : x));
+            if (REDUCE) {
+                acc.a.add(fabsf(x - old));
+                acc.b.add(d ? 0.f : x);
+            }
             __stcg(a.rank_p + r, x);
             if (a.swap) __stcg(cout + r, d ? __fdiv_rn(x, (float)d) : 0.f);
         };
@@ -266,7 +255,7 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
             if (mine && sl == 0) emit(r, s, old);
         }
         for (uint32_t r = x0 + tid; r < x1; r += EG_PRS_THREADS) emit(r, 0.f, last_rank(r));
-        if (REDUCE) prs_block_sum(acc, s_sum, a.part + ((it + 1) & 1) * G + b);
+        if (REDUCE) eg_store_sum(eg_block_sum(acc, s_sum), a.part + ((it + 1) & 1) * G + b);
     }
     for (uint32_t v = v0 + tid; v < v1; v += EG_PRS_THREADS) a.rank[v] = __ldcg(a.rank_p + __ldg(a.perm + v));
 }

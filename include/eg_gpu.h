@@ -144,9 +144,10 @@ void *eg_graph_device_ptr(eg_graph *g, int which);
  * reproduces pagerank_simple's pull mode, where prev is never updated.
  * deg_multiplier=2 reproduces the doubled degrees of the grid load modes
  * (init_all.c:851-852).  prev_init < 0 means 1/n (the reference uses 0.15).
- * dangling=1 spreads the mass of out-degree-0 vertices uniformly (FP64
- * reduction on the device); 0 drops it like the reference.
- * tolerance > 0 stops once the FP64 L1 change between iterates is below it. */
+ * dangling=1 spreads the mass of out-degree-0 vertices uniformly; 0 drops it
+ * like the reference.  tolerance > 0 stops once the L1 change between iterates
+ * is below it.  Both sums are kept as fp32 words with their rounding errors
+ * (about 70 bits) and widened to FP64 once. */
 typedef struct {
     int iterations;
     float damping;
@@ -173,8 +174,8 @@ typedef struct {
 } eg_pr_opts;
 typedef struct {
     int iterations_run;
-    double residual;      /* FP64 L1 change of the last iteration (if computed) */
-    double dangling_mass; /* FP64 mass on out-degree-0 vertices, last iterate */
+    double residual;      /* L1 change of the last iteration (if computed) */
+    double dangling_mass; /* mass on out-degree-0 vertices, last iterate */
     float ms;             /* device time of the iterations */
     float row_kernel_ms;  /* mean device time of one row-sum kernel launch (up to
                              the first 8 iterations; 0 when use_graph; small
