@@ -27,6 +27,15 @@ struct PprQ {  // per-query state (device)
 __device__ __forceinline__ float4 eg_f4add(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
+// Eight rows' sum.  Long sums take them eight by eight: a chain of an addition
+// per eight entries rounds less (511 equal entries one by one: off by 7.6e-6 of
+// the sum, this way by 5e-8).
+__device__ __forceinline__ float4 eg_f4sum8(const float4 (&x)[8]) {
+    float4 s = x[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++) s = eg_f4add(s, x[i]);
+    return s;
+}
 __device__ __forceinline__ float4 eg_f4shfl(unsigned mask, float4 v, int src) {
     return make_float4(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src), __shfl_sync(mask, v.z, src),
                        __shfl_sync(mask, v.w, src));
@@ -40,8 +49,8 @@ __device__ __forceinline__ float4 eg_f4shfl(unsigned mask, float4 v, int src) {
 // The warp is four groups of 8 lanes; lane s of a group holds queries
 // 4s..4s+3 (one 16-byte load brings a group a whole 128-byte row of X), and a
 // group takes one item, 8 entries per step with their 8 row loads in flight.
-// An item is summed in entry order, so a query's bits depend on the graph
-// alone.  Items of a warp have nearly equal lengths and no entry needs a row
+// An item is summed in entry order, eight entries at a time, so a query's bits
+// depend on the graph alone.  Items of a warp have nearly equal lengths and no entry needs a row
 // id or a test for the row's end; the next item's place is loaded while the
 // current one is summed.  Bound by the latency of the L2 row reads (a
 // sweep of undirected RMAT-20: 249 us, 15 TB/s of rows; 413 when each warp
@@ -89,17 +98,18 @@ __global__ void __launch_bounds__(256, EG_PPR_MINB) k_ppr_rows(const uint32_t *_
 #pragma unroll
                 for (int q = 0; q < 8; q++)
                     xv[q] = __ldg(X4 + (uint64_t)__shfl_sync(EG_FULL_MASK, my_c, q, 8) * (EG_PPR_LANES / 4));
-#pragma unroll
-                for (int q = 0; q < 8; q++) acc = eg_f4add(acc, xv[q]);
+                acc = eg_f4add(acc, eg_f4sum8(xv));
             } else {
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
                     const uint32_t u = __shfl_sync(EG_FULL_MASK, my_c, q, 8);
                     xv[q] = b + q < cur.len ? __ldg(X4 + (uint64_t)u * (EG_PPR_LANES / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
+                float4 s = xv[0];
 #pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (b + q < cur.len) acc = eg_f4add(acc, xv[q]);
+                for (int q = 1; q < 8; q++)
+                    if (b + q < cur.len) s = eg_f4add(s, xv[q]);
+                acc = eg_f4add(acc, s);
             }
             my_c = next_c;
         }
@@ -130,10 +140,8 @@ __global__ void __launch_bounds__(256) k_ppr_fixup(const uint4 *__restrict__ mul
         float4 x[EG_PPR_FIXUP];
 #pragma unroll
         for (uint32_t i = 0; i < EG_PPR_FIXUP; i++)
-            if (k + i < k1) x[i] = __ldcg(P4 + (uint64_t)(k + i) * (EG_PPR_LANES / 4));
-#pragma unroll
-        for (uint32_t i = 0; i < EG_PPR_FIXUP; i++)
-            if (k + i < k1) acc = eg_f4add(acc, x[i]);
+            x[i] = k + i < k1 ? __ldcg(P4 + (uint64_t)(k + i) * (EG_PPR_LANES / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        acc = eg_f4add(acc, eg_f4sum8(x));
     }
     float4 tot = eg_f4shfl(EG_FULL_MASK, acc, (int)sl);
 #pragma unroll
