@@ -1005,31 +1005,31 @@ __global__ void __launch_bounds__(256) k_row_runs(const uint32_t *__restrict__ r
                                                   uint32_t *last) {
     const uint32_t nq = (uint32_t)(((uint64_t)m + 3) >> 2);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const uint32_t b = q * 4;
+        const uint32_t b = q * 4, left = m - b;  // b + 4 may not fit 32 bits
         uint32_t prev = b ? __ldg(rid + b - 1) : 0u;
         uint4 x;
-        if (b + 4 <= m) x = __ldg(reinterpret_cast<const uint4 *>(rid) + q);
+        if (left >= 4) x = __ldg(reinterpret_cast<const uint4 *>(rid) + q);
         else {
             x.x = __ldg(rid + b);
-            x.y = b + 1 < m ? __ldg(rid + b + 1) : 0u;
-            x.z = b + 2 < m ? __ldg(rid + b + 2) : 0u;
+            x.y = left > 1 ? __ldg(rid + b + 1) : 0u;
+            x.z = left > 2 ? __ldg(rid + b + 2) : 0u;
             x.w = 0u;
         }
         const uint32_t r[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (b + i >= m) break;
+        for (uint32_t i = 0; i < 4; i++) {
+            if (i >= left) break;
             if (b + i == 0 || r[i] != prev) {
                 first[r[i]] = b + i;
                 if (b + i) last[prev] = b + i;
             }
             prev = r[i];
         }
-        if (b + 4 >= m) last[prev] = m;
+        if (left <= 4) last[prev] = m;
     }
 }
 __global__ void k_run_lengths(const uint32_t *__restrict__ first, uint32_t n, uint32_t *last_to_len) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    for (uint64_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
         last_to_len[v] -= first[v];
 }
 
