@@ -395,18 +395,19 @@ __global__ void __launch_bounds__(256) k_sssp_push(const uint4 *__restrict__ que
             uint32_t v[EG_SSSP_STEP], nd[EG_SSSP_STEP], wt[EG_SSSP_STEP];
 #pragma unroll
             for (int k = 0; k < EG_SSSP_STEP; k++) {
-                const uint32_t x0 = p + 32 * k, x = x0 + lane;
+                const uint32_t x0 = p + 32 * k;
                 const uint32_t starts =
                     __reduce_or_sync(EG_FULL_MASK, q.x - x0 < 32u ? 1u << (q.x - x0) : 0u);
                 const uint32_t o = __popc(__ballot_sync(EG_FULL_MASK, q.x < x0)) - 1 + __popc(starts & le);
-                const uint32_t at = x + __shfl_sync(EG_FULL_MASK, q.y, o);
+                const uint32_t at = x0 + lane + __shfl_sync(EG_FULL_MASK, q.y, o);
+                const bool on = stop - p > 32u * k + lane;  // x0 + lane may not fit 32 bits
                 nd[k] = __shfl_sync(EG_FULL_MASK, q.z, o);
-                v[k] = x < stop ? __ldg(col + at) : 0u;
-                wt[k] = x < stop ? __ldg(wts + at) : 0u;
+                v[k] = on ? __ldg(col + at) : 0u;
+                wt[k] = on ? __ldg(wts + at) : 0u;
             }
             uint32_t cur[EG_SSSP_STEP];
 #pragma unroll
-            for (int k = 0; k < EG_SSSP_STEP; k++) cur[k] = p + 32 * k + lane < stop ? __ldca(dist + v[k]) : 0u;
+            for (int k = 0; k < EG_SSSP_STEP; k++) cur[k] = stop - p > 32u * k + lane ? __ldca(dist + v[k]) : 0u;
 #pragma unroll
             for (int k = 0; k < EG_SSSP_STEP; k++) {
                 nd[k] = w.add(nd[k], wt[k]);
@@ -431,7 +432,7 @@ __global__ void k_count_reached(const uint32_t *__restrict__ dist, uint64_t len,
 
 __global__ void k_edge_weights(const uint32_t *__restrict__ rid, const uint32_t *__restrict__ col, uint32_t m,
                                WRule w, uint32_t *__restrict__ out) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
+    for (uint64_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
         out[p] = w.weight(__ldg(rid + p), __ldg(col + p));
 }
 

@@ -31,3 +31,38 @@ def test_row_starts(m):
     assert np.array_equal(np.diff(ptr.astype(np.int64)), deg)
     assert np.all(np.abs(deg - m / n) < 8 * (m / n) ** 0.5)  # uniform draws
     ctx.close()
+
+
+def test_sssp_round_over_all_entries():
+    """One round lists all entries but two: vertices 5 and 20 are reached at
+    distances 5 and 0, their lists fill the places up to 2^32 - 4."""
+    import torch
+
+    import everythinggraph_gb300 as eg
+
+    need(130)
+    n, m = 50, 2 ** 32 - 2
+    pairs = torch.empty((m, 2), dtype=torch.int32, device="cuda")
+    pairs[:, 0] = 5
+    pairs[:, 1] = 30
+    for i in range(1, 8):  # the first entries of 5's list, which places past 2^32 would wrap to
+        pairs[i::1 << 10, 1] = 30 + i
+    pairs[-2, 0], pairs[-2, 1] = 10, 5
+    pairs[-1, 0], pairs[-1, 1] = 10, 20
+    pairs[-102:-2, 0] = 20
+    pairs[-102:-2, 1] = 40 + torch.arange(100, dtype=torch.int32, device="cuda") % 10
+    torch.cuda.synchronize()
+    ctx = eg.Context(0)
+    g = ctx.from_device_pairs(n, pairs.data_ptr(), m)
+    ctx.sync()
+    del pairs
+    torch.cuda.empty_cache()
+    g.build(eg.CSR)
+    dist, st = g.sssp(10, eg.weights("ref"))  # u % 10 + v % 10
+    ref = np.full(n, eg.UNREACHED_SSSP, dtype=np.uint32)
+    ref[10], ref[5], ref[20] = 0, 5, 0
+    ref[30:38] = 10 + np.arange(8)
+    ref[40:50] = np.arange(10)
+    assert np.array_equal(dist, ref)
+    assert st.relaxations == m
+    ctx.close()
