@@ -49,8 +49,9 @@ def test_sssp_round_over_all_entries():
         pairs[i::1 << 10, 1] = 30 + i
     pairs[-2, 0], pairs[-2, 1] = 10, 5
     pairs[-1, 0], pairs[-1, 1] = 10, 20
-    pairs[-102:-2, 0] = 20
-    pairs[-102:-2, 1] = 40 + torch.arange(100, dtype=torch.int32, device="cuda") % 10
+    z = 1 << 20  # more than a warp's share: the last warp's window holds vertex 20 alone
+    pairs[-2 - z:-2, 0] = 20
+    pairs[-2 - z:-2, 1] = 40 + torch.arange(z, dtype=torch.int32, device="cuda") % 10
     torch.cuda.synchronize()
     ctx = eg.Context(0)
     g = ctx.from_device_pairs(n, pairs.data_ptr(), m)
