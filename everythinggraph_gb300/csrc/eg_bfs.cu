@@ -130,7 +130,7 @@ static int bfs_core(eg_graph *g, uint32_t root, const eg_bfs_opts &o, int slot, 
               in_adj ? bp<uint32_t>(in_adj->col) : nullptr, first, first ? first + first_words(n) : nullptr,
               bp<uint32_t>(g->out_deg), n, nw, root, o.direction, divisor > 0 ? (double)g->m / divisor : 0.0, level, parent,
               bits, bits + nw4, {bits + 2 * nw4, bits + 3 * nw4}, reinterpret_cast<uint4 *>(wk), st};
-    const uint64_t want = g->m / EG_BFSL_SHARE + 1, most = (uint64_t)ctx->sm_count * EG_BFSL_B;
+    const uint64_t want = (g->m + n) / EG_BFSL_SHARE + 1, most = (uint64_t)ctx->sm_count * EG_BFSL_B;
     void *args[] = {&a};
     EG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     EG_CUDA(cudaLaunchCooperativeKernel(parent ? (const void *)k_bfs_loop<true> : (const void *)k_bfs_loop<false>,

@@ -29,7 +29,10 @@
 #define EG_BFSL_T 512      // threads per CTA
 #define EG_BFSL_B 2        // CTAs per SM
 #define EG_BFSL_STEP 4     // places per lane in flight in a push
-#define EG_BFSL_SHARE 4096u  // entries per CTA below a full grid
+// Entries and vertices per CTA below a full grid.  The vertices count for the
+// start values and the passes over the bitmaps: n = 16.8 M with 4 K entries,
+// grid by the entries alone (3 CTAs) 1456 us, by both 59.
+#define EG_BFSL_SHARE 4096u
 #define EG_BFSL_ALONE 8    // 16-byte steps of a pull's list that one lane takes
 #define EG_NO_VERTEX 0xffffffffu
 
