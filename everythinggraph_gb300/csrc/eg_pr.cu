@@ -642,7 +642,9 @@ static bool pr_small(const eg_graph *g, const eg_pr_opts &o) {
 static int pr_run_small(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr_stats *stats) {
     eg_ctx *ctx = g->ctx;
     const uint32_t n = g->n, m = (uint32_t)g->m;
-    const uint32_t want = eg_div_up(m, EG_PRS_SHARE), G = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
+    // a share of the entries each, and at most a vertex per thread
+    const uint32_t by_m = eg_div_up(m, EG_PRS_SHARE), by_n = eg_div_up(n, EG_PRS_THREADS);
+    const uint32_t want = by_m > by_n ? by_m : by_n, G = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
     for (eg_buf *b : {&g->rank, &g->rank_p, &g->contrib0, &g->contrib1}) EG_TRY(eg_buf_ensure(ctx, *b, (uint64_t)n * 4));
     EG_TRY(eg_buf_ensure(ctx, g->pr_part, 2ull * G * sizeof(eg_sum2)));
     eg_pr_dev *st = bp<eg_pr_dev>(g->pr_stats);

@@ -36,7 +36,7 @@
 #define EG_PRS_GROUP 128u
 #define EG_PRS_WARP 4096u
 #define EG_PRS_MAX_LONG 64u
-#define EG_PRS_SHARE 2048u          // entries per CTA below a full grid
+#define EG_PRS_SHARE 2048u          // entries per CTA below a full grid (and EG_PRS_THREADS vertices)
 
 namespace {
 

@@ -37,3 +37,17 @@ def test_bfs(n):
     ctx.close()
     print(t)
     assert t[0] <= t[1], t
+
+
+@pytest.mark.parametrize("n", [40960, 1 << 18])
+@pytest.mark.parametrize("tolerance", [0.0, 1e-30])
+def test_pagerank(n, tolerance):
+    ctx = __import__("everythinggraph_gb300").Context(0)
+    t = []
+    for m in (1000, None):
+        g = graph(ctx, n, m)
+        t.append(best(lambda: g.pagerank(iterations=20, tolerance=tolerance, dangling=tolerance > 0, copy_out=False)))
+        g.free()
+    ctx.close()
+    print(t)
+    assert t[0] <= t[1], t
