@@ -628,9 +628,6 @@ static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st
     return EG_OK;
 }
 
-// Shared by eg_pagerank and eg_ppr: the iterations over the relabelled CSC,
-// then the ranks back in the original vertex order.  `ps` (in relabelled
-// ids) selects the personalised teleport; its total multiplicity divides it.
 // Whether a run goes to k_pr_small: plain PageRank on the default schedule, of
 // a size where its one launch is faster than the launches per iteration (the
 // figures are beside the kernel).
@@ -683,6 +680,9 @@ static int pr_run_small(eg_graph *g, const eg_pr_opts &o, float *rank_out, eg_pr
     return EG_OK;
 }
 
+// Shared by eg_pagerank and eg_ppr: the iterations over the relabelled CSC,
+// then the ranks back in the original vertex order.  `ps` (in relabelled
+// ids) selects the personalised teleport; its total multiplicity divides it.
 static int pr_run(eg_graph *g, const eg_pr_opts &o, const PprSeeds &ps, uint32_t seed_total, float *rank_out,
                   eg_pr_stats *stats) {
     eg_ctx *ctx = g->ctx;
@@ -832,11 +832,22 @@ extern "C" int eg_graph_tune(eg_graph *g, eg_tune_result *out) {
     r.ncand = EG_PR_CANDS;
     int best = 0;
     g->pr_kernel = 0;
+    g->row_cfg = 0;
+    // where schedule 0 runs all iterations in one launch, the candidates are
+    // compared by the time of a whole iteration (10,007 vertices: the launches
+    // per iteration of any other schedule 243 us for ten, the one launch 62)
+    const bool whole = pr_small(g, o);
+    auto run = [&](eg_pr_stats *st) -> int {
+        if (pr_small(g, o)) return pr_run_small(g, o, nullptr, st);
+        EG_TRY(pr_run(g, o, none, 0, nullptr, st));
+        if (whole) st->row_kernel_ms = st->ms / (float)o.iterations;
+        return EG_OK;
+    };
     for (int c = 0; c < EG_ROW_CFGS; c++) {
         g->row_cfg = c;
         eg_pr_stats st;
-        EG_TRY(pr_run(g, o, none, 0, nullptr, &st));  // warm-up (caches, carries)
-        EG_TRY(pr_run(g, o, none, 0, nullptr, &st));
+        EG_TRY(run(&st));  // warm-up (caches, carries)
+        EG_TRY(run(&st));
         r.tile_entries[c] = kRowCfg[c].tile;
         r.entries_per_lane[c] = kRowCfg[c].u;
         r.prefetch[c] = kRowCfg[c].pf;
@@ -864,8 +875,8 @@ extern "C" int eg_graph_tune(eg_graph *g, eg_tune_result *out) {
         EG_TRY(prc);
         g->pr_kernel = 1;
         eg_pr_stats st;
-        EG_TRY(pr_run(g, o, none, 0, nullptr, &st));
-        EG_TRY(pr_run(g, o, none, 0, nullptr, &st));
+        EG_TRY(run(&st));
+        EG_TRY(run(&st));
         r.ms[c] = st.row_kernel_ms;
         if (st.row_kernel_ms < r.ms[best]) {
             r.chosen = c;

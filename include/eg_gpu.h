@@ -213,7 +213,9 @@ typedef struct {
     int prefetch[EG_ROW_SCHEDULES_MAX];
     int min_blocks[EG_ROW_SCHEDULES_MAX];
     int cache_hint[EG_ROW_SCHEDULES_MAX];
-    float ms[EG_ROW_SCHEDULES_MAX]; /* mean row-kernel time per iteration */
+    float ms[EG_ROW_SCHEDULES_MAX]; /* mean row-kernel time per iteration; on
+                                 graphs that schedule 0 runs in one launch, the
+                                 time of a whole iteration */
     /* 0: a row-kernel schedule; k > 0: PageRank's partition kernel over
      * partitions of 2^k rows (the last candidate) */
     int partition_log2[EG_ROW_SCHEDULES_MAX];
