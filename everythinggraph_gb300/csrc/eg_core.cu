@@ -217,11 +217,13 @@ int eg_dmalloc(eg_ctx *c, void **p, uint64_t bytes) {
             return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
                            (unsigned long long)c->in_use, (unsigned long long)bytes, (unsigned long long)c->budget);
     }
-    // the smallest kept block that fits with at most an eighth to spare
+    // the smallest kept block that fits with at most an eighth to spare (none
+    // under a budget: what is held would be more than what is counted)
+    const uint64_t most = c->budget ? bytes : bytes + bytes / 8;
     size_t best = c->kept.size();
     for (size_t i = 0; i < c->kept.size(); i++) {
         const uint64_t b = c->kept[i].bytes;
-        if (b >= bytes && b <= bytes + bytes / 8 && (best == c->kept.size() || b < c->kept[best].bytes)) best = i;
+        if (b >= bytes && b <= most && (best == c->kept.size() || b < c->kept[best].bytes)) best = i;
     }
     if (best < c->kept.size()) {
         if (c->kept_busy) {  // as after cudaFree: nothing queued anywhere still uses it
