@@ -124,6 +124,15 @@ class Context:
         return lib().eg_bytes_in_use(self._h)
 
     @property
+    def bytes_kept(self):
+        """Device memory kept for the next buffers (eg_bytes_kept)."""
+        return lib().eg_bytes_kept(self._h)
+
+    def trim(self):
+        """Gives the kept memory back to the device."""
+        L.check(lib().eg_trim(self._h))
+
+    @property
     def kernel_launches(self):
         return lib().eg_kernel_launches(self._h)
 

@@ -117,6 +117,8 @@ SIGNATURES = {
     "eg_stream": (c_void_p, [c_void_p]),
     "eg_sync": (c_int, [c_void_p]),
     "eg_bytes_in_use": (c_u64, [c_void_p]),
+    "eg_bytes_kept": (c_u64, [c_void_p]),
+    "eg_trim": (c_int, [c_void_p]),
     "eg_kernel_launches": (c_u64, [c_void_p]),
     "eg_graph_from_pairs": (c_int, [c_void_p, c_void_p, c_u64, c_u32, ctypes.c_uint, P(c_void_p)]),
     "eg_graph_from_device_pairs": (c_int, [c_void_p, c_void_p, c_u64, c_u32, ctypes.c_uint, P(c_void_p)]),

@@ -12,6 +12,8 @@
 
 #include <time.h>
 
+#include <mutex>
+
 #include "eg_internal.cuh"
 
 // ============================================================== errors
@@ -30,6 +32,10 @@ extern "C" const char *eg_last_error(void) { return g_err; }
 extern "C" const char *eg_version(void) { return "everythinggraph_gb300 0.1 (sm_103a)"; }
 
 // ============================================================== context
+// Every open context, for drop_all_kept.  Taken before a context's own lock.
+static std::mutex g_open_lock;
+static std::vector<eg_ctx *> g_open;
+
 extern "C" int eg_open(int device, uint64_t hbm_budget_bytes, eg_ctx **out) {
     if (!out) return eg_fail(EG_EINVAL, "eg_open: out is NULL");
     *out = nullptr;
@@ -50,6 +56,8 @@ extern "C" int eg_open(int device, uint64_t hbm_budget_bytes, eg_ctx **out) {
     for (cudaEvent_t &e : c->evk) EG_CUDA(cudaEventCreate(&e));
     EG_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     for (cudaEvent_t &e : c->ev_out) EG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    std::lock_guard<std::mutex> hold(g_open_lock);
+    g_open.push_back(c);
     *out = c;
     return EG_OK;
 }
@@ -152,10 +160,15 @@ extern "C" int eg_host_free(void *p) {
 static void drop_scratch(eg_ctx *c);
 extern "C" int eg_close(eg_ctx *c) {
     if (!c) return EG_OK;
-    if (c->live_graphs > 0) return eg_fail(EG_EINVAL, "eg_close: %d graphs are still open", c->live_graphs);
+    if (c->live_graphs > 0) return eg_fail(EG_EINVAL, "eg_close: %d graphs are still open", c->live_graphs.load());
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaStreamSynchronize(c->copy_stream);
+    {
+        std::lock_guard<std::mutex> hold(g_open_lock);
+        for (size_t i = 0; i < g_open.size(); i++)
+            if (g_open[i] == c) g_open.erase(g_open.begin() + i--);
+    }
     drop_scratch(c);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
@@ -182,15 +195,20 @@ extern "C" uint64_t eg_kernel_launches(eg_ctx *c) { return c ? c->launches : 0; 
 // to EG_KEEP_BYTES of them, oldest given back to the driver first: a layout
 // build allocates and frees about 30 bytes per entry, and cudaMalloc and
 // cudaFree of 512 MB take 156 and 282 us here (2 GB: 0.6 and 1.0 ms).  Build
-// of undirected RMAT-22 from device pairs: 9.6 ms without, 5.5 ms with
-// kept blocks.  Kept blocks
-// never make an allocation fail: they go back to the driver when the budget
-// or the device has no room beside them, and with the context.
+// of undirected RMAT-22 from device pairs beside another graph: 9.6 ms without,
+// 5.5 ms with kept blocks.
+//
+// They go back to the driver with the context's last graph, by eg_trim, when
+// the budget or the device has no room beside them (for an allocation or a
+// CUDA graph of any context of the process), and once less than an eighth of
+// the device's memory is free (asked every EG_KEEP_ASK bytes: 5 us and more).
 #define EG_KEEP_BYTES (8ull << 30)
 #define EG_KEEP_BLOCKS 64u
 #define EG_KEEP_MIN 65536ull  // smaller blocks go straight back
+#define EG_KEEP_ASK (1ull << 30)
 
 static void drop_kept(eg_ctx *c, uint64_t down_to) {
+    std::lock_guard<std::recursive_mutex> hold(c->mem);
     size_t k = 0;
     while (k < c->kept.size() && c->kept_bytes > down_to) {
         cudaFree(c->kept[k].p);  // waits for the device
@@ -202,58 +220,100 @@ static void drop_kept(eg_ctx *c, uint64_t down_to) {
 
 // Everything the context holds beyond the live buffers of its graphs.
 static void drop_scratch(eg_ctx *c) {
+    std::lock_guard<std::recursive_mutex> hold(c->mem);
     cudaStreamSynchronize(c->stream);
     eg_buf_free(c, c->sort_ws);
     eg_buf_free(c, c->scan_ws);
     drop_kept(c, 0);
 }
 
-int eg_dmalloc(eg_ctx *c, void **p, uint64_t bytes) {
-    *p = nullptr;
-    if (bytes == 0) return EG_OK;
-    if (c->budget && c->in_use + c->kept_bytes + bytes > c->budget) {
-        drop_scratch(c);
-        if (c->in_use + bytes > c->budget)
-            return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
-                           (unsigned long long)c->in_use, (unsigned long long)bytes, (unsigned long long)c->budget);
+// The device has no room: this context's scratch and every context's kept
+// blocks on its device.  The calling thread holds no context's lock.
+static void drop_all_kept(eg_ctx *c) {
+    drop_scratch(c);
+    std::lock_guard<std::mutex> hold(g_open_lock);
+    for (eg_ctx *o : g_open)
+        if (o->device == c->device) drop_kept(o, 0);
+}
+
+extern "C" int eg_trim(eg_ctx *c) {
+    if (!c) return eg_fail(EG_EINVAL, "eg_trim: NULL context");
+    EG_CUDA(cudaSetDevice(c->device));
+    drop_scratch(c);
+    return EG_OK;
+}
+extern "C" uint64_t eg_bytes_kept(eg_ctx *c) {
+    if (!c) return 0;
+    std::lock_guard<std::recursive_mutex> hold(c->mem);
+    return c->kept_bytes;
+}
+
+int eg_graph_instantiate(eg_ctx *c, cudaGraphExec_t *exec, cudaGraph_t graph) {
+    cudaError_t e = cudaGraphInstantiate(exec, graph, 0);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        drop_all_kept(c);
+        e = cudaGraphInstantiate(exec, graph, 0);
     }
-    // the smallest kept block that fits with at most an eighth to spare (none
-    // under a budget: what is held would be more than what is counted)
+    EG_CUDA(e);
+    return EG_OK;
+}
+
+// A kept block in *p, if one fits: the smallest, with at most an eighth to
+// spare (none under a budget: what is held would be more than what is counted).
+static int take_kept(eg_ctx *c, void **p, uint64_t bytes) {
     const uint64_t most = c->budget ? bytes : bytes + bytes / 8;
     size_t best = c->kept.size();
     for (size_t i = 0; i < c->kept.size(); i++) {
         const uint64_t b = c->kept[i].bytes;
         if (b >= bytes && b <= most && (best == c->kept.size() || b < c->kept[best].bytes)) best = i;
     }
-    if (best < c->kept.size()) {
-        if (c->kept_busy) {  // as after cudaFree: nothing queued anywhere still uses it
-            EG_CUDA(cudaDeviceSynchronize());
-            c->kept_busy = false;
-        }
-        *p = c->kept[best].p;
-        c->kept_bytes -= c->kept[best].bytes;
-        c->live[*p] = c->kept[best].bytes;
-        c->kept.erase(c->kept.begin() + best);
-        c->in_use += bytes;
-        return EG_OK;
+    if (best == c->kept.size()) return EG_OK;
+    if (c->kept_busy) {  // as after cudaFree: nothing queued anywhere still uses it
+        EG_CUDA(cudaDeviceSynchronize());
+        c->kept_busy = false;
     }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && (c->kept_bytes || c->sort_ws.p || c->scan_ws.p)) {
-        cudaGetLastError();
-        drop_scratch(c);
-        e = cudaMalloc(p, bytes);
-    }
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-        return eg_fail(EG_ENOMEM, "cudaMalloc(%llu): %s", (unsigned long long)bytes, cudaGetErrorString(e));
-    }
-    c->live[*p] = bytes;
+    *p = c->kept[best].p;
+    c->kept_bytes -= c->kept[best].bytes;
+    c->live[*p] = c->kept[best].bytes;
+    c->kept.erase(c->kept.begin() + best);
     c->in_use += bytes;
     return EG_OK;
 }
+
+int eg_dmalloc(eg_ctx *c, void **p, uint64_t bytes) {
+    *p = nullptr;
+    if (bytes == 0) return EG_OK;
+    cudaError_t e = cudaSuccess;
+    for (int attempt = 0; attempt < 2; attempt++) {
+        {
+            std::lock_guard<std::recursive_mutex> hold(c->mem);
+            if (c->budget && c->in_use + c->kept_bytes + bytes > c->budget) {
+                drop_scratch(c);
+                if (c->in_use + bytes > c->budget)
+                    return eg_fail(EG_ENOMEM, "HBM budget exceeded: %llu in use + %llu requested > %llu",
+                                   (unsigned long long)c->in_use, (unsigned long long)bytes,
+                                   (unsigned long long)c->budget);
+            }
+            EG_TRY(take_kept(c, p, bytes));
+            if (*p) return EG_OK;
+            e = cudaMalloc(p, bytes);
+            if (e == cudaSuccess) {
+                c->live[*p] = bytes;
+                c->in_use += bytes;
+                return EG_OK;
+            }
+        }
+        cudaGetLastError();
+        *p = nullptr;
+        if (e != cudaErrorMemoryAllocation) break;
+        if (attempt == 0) drop_all_kept(c);
+    }
+    return eg_fail(EG_ENOMEM, "cudaMalloc(%llu): %s", (unsigned long long)bytes, cudaGetErrorString(e));
+}
 void eg_dfree(eg_ctx *c, void *p, uint64_t bytes) {
     if (!p) return;
+    std::lock_guard<std::recursive_mutex> hold(c->mem);
     c->in_use -= bytes;
     const auto it = c->live.find(p);
     const uint64_t size = it == c->live.end() ? 0 : it->second;
@@ -261,6 +321,15 @@ void eg_dfree(eg_ctx *c, void *p, uint64_t bytes) {
     if (size < EG_KEEP_MIN || size > EG_KEEP_BYTES) {
         cudaFree(p);
         return;
+    }
+    if (c->unasked += size; c->unasked >= EG_KEEP_ASK) {
+        c->unasked = 0;
+        size_t room = 0, all = 0;
+        if (cudaMemGetInfo(&room, &all) != cudaSuccess || room < all / 8) {
+            cudaFree(p);
+            drop_kept(c, 0);
+            return;
+        }
     }
     drop_kept(c, EG_KEEP_BYTES - size);
     if (c->kept.size() >= EG_KEEP_BLOCKS) drop_kept(c, c->kept_bytes - c->kept[0].bytes);
@@ -484,8 +553,8 @@ extern "C" void eg_graph_free(eg_graph *g) {
         if (bg->exec) cudaGraphExecDestroy(bg->exec);
         if (bg->graph) cudaGraphDestroy(bg->graph);
     }
-    c->live_graphs--;
     delete g;
+    if (--c->live_graphs == 0) drop_scratch(c);
 }
 
 // ============================================================== scan
@@ -1108,7 +1177,7 @@ static int build_adj_pair(eg_graph *g, bool want_csc) {
         BTRY(rows_from_rid(ctx, bp<uint32_t>(g->csc.rid), M, n, bp<uint32_t>(g->in_deg), bp<uint32_t>(g->csc.ptr)));
         g->built |= EG_LAYOUT_CSC;
         g->first_in_src = nullptr;
-            g->relabeled = false;  // so do PageRank's relabelled copy
+        g->relabeled = false;  // so does PageRank's relabelled copy
         g->ppr_planned = false;
         g->sb.blocks = 0;  // the source-blocked copies follow the CSC
         g->sb.shift = 0;

@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+#include <mutex>
 #include <unordered_map>
 #include <vector>
 
@@ -65,15 +67,17 @@ struct eg_ctx {
     void *h_pinned_dev;  // the same memory as the device addresses it
     cudaEvent_t ev0, ev1;
     cudaEvent_t evk[2 * EG_KEV];  // begin/end pairs around single kernel launches
-    int live_graphs;              // eg_close refuses while graphs are alive
+    std::atomic<int> live_graphs;  // eg_close refuses while graphs are alive
     cudaStream_t copy_stream;     // device-to-host copies overlapped with the next traversal
     cudaEvent_t ev_out[2 * EG_OUT_SLOTS];  // [slot]: outputs ready, [EG_OUT_SLOTS + slot]: copied out
     uint32_t rb_seq = 0;                   // eg_readback_wait: the last flag value asked for
     // eg_dmalloc's kept blocks, oldest first (their bytes are not in in_use),
     // whether one of them may still be in use by work queued before it was
-    // given back, and the sizes of the live blocks
+    // given back, and the sizes of the live blocks; `mem` guards them and
+    // in_use (a finaliser may free a graph on another thread)
+    std::recursive_mutex mem;
     std::vector<eg_block> kept;
-    uint64_t kept_bytes = 0;
+    uint64_t kept_bytes = 0, unasked = 0;  // unasked: kept since the device's free memory was asked for
     bool kept_busy = false;
     std::unordered_map<void *, uint64_t> live;
     eg_buf sort_ws, scan_ws;  // radix sort counts, scan sums: used on `stream` only, kept between calls
@@ -84,6 +88,8 @@ struct eg_ctx {
 int eg_dmalloc(eg_ctx *ctx, void **p, uint64_t bytes);
 void eg_dfree(eg_ctx *ctx, void *p, uint64_t bytes);
 
+// cudaGraphInstantiate, once more without kept blocks when memory is short.
+int eg_graph_instantiate(eg_ctx *ctx, cudaGraphExec_t *exec, cudaGraph_t graph);
 int eg_buf_ensure(eg_ctx *ctx, eg_buf &b, uint64_t bytes);  // grows (contents lost)
 // Small device-to-host readback into ctx->h_pinned (host_dst lies in it) by a
 // one-warp kernel on `st` instead of a copy engine, so that it does not queue

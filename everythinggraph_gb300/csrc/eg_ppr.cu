@@ -89,7 +89,7 @@ int ppr_graph_build(eg_graph *g, const void *const key[8], uint32_t fin_blocks, 
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &body);
     if (ce != cudaSuccess) return eg_fail(EG_ECUDA, "batched PageRank capture: %s", cudaGetErrorString(ce));
     cudaGraphExec_t exec = nullptr;
-    EG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    EG_TRY(eg_graph_instantiate(ctx, &exec, graph));
     bg.exec = exec;
     for (int i = 0; i < 8; i++) bg.key[i] = key[i];
     return EG_OK;

@@ -623,7 +623,7 @@ static int pr_graph(eg_graph *g, const eg_pr_opts &o, bool reduce, eg_pr_dev *st
     }
     if (e != cudaSuccess) return eg_fail(EG_ECUDA, "PageRank capture: %s", cudaGetErrorString(e));
     g->prg.graph = gr;
-    EG_CUDA(cudaGraphInstantiate(&g->prg.exec, gr, 0));
+    EG_TRY(eg_graph_instantiate(ctx, &g->prg.exec, gr));
     memcpy(g->prk, key, sizeof(key));
     return EG_OK;
 }

@@ -517,7 +517,7 @@ static int sssp_graph_build(eg_graph *g, const void *const key[8], const uint32_
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &body);
     if (ce != cudaSuccess) return eg_fail(EG_ECUDA, "SSSP capture: %s", cudaGetErrorString(ce));
     cudaGraphExec_t exec = nullptr;
-    EG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    EG_TRY(eg_graph_instantiate(ctx, &exec, graph));
     bg.exec = exec;
     for (int i = 0; i < 8; i++) bg.key[i] = key[i];
     return EG_OK;
@@ -957,7 +957,7 @@ static int msssp_graph_build(eg_graph *g, const void *const key[8], const uint32
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &body);
     if (ce != cudaSuccess) return eg_fail(EG_ECUDA, "batched SSSP capture: %s", cudaGetErrorString(ce));
     cudaGraphExec_t exec = nullptr;
-    EG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    EG_TRY(eg_graph_instantiate(ctx, &exec, graph));
     bg.exec = exec;
     for (int i = 0; i < 8; i++) bg.key[i] = key[i];
     return EG_OK;

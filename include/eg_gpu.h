@@ -54,6 +54,12 @@ int eg_close(eg_ctx *ctx); /* EG_EINVAL (context kept) while graphs are open:
 void *eg_stream(eg_ctx *ctx);
 int eg_sync(eg_ctx *ctx);
 uint64_t eg_bytes_in_use(eg_ctx *ctx);
+/* Device memory that freed buffers left behind and the context keeps for its
+ * next ones (at most 8 GiB, not in eg_bytes_in_use, within the budget).  It
+ * goes back with the context's last graph, when any context of the process has
+ * no room beside it, or by eg_trim (for other users of the device). */
+uint64_t eg_bytes_kept(eg_ctx *ctx);
+int eg_trim(eg_ctx *ctx);
 /* Number of kernels this context has launched so far. */
 uint64_t eg_kernel_launches(eg_ctx *ctx);
 
