@@ -125,10 +125,12 @@ static int bfs_core(eg_graph *g, uint32_t root, const eg_bfs_opts &o, int slot, 
     int32_t *level = bp<int32_t>(lbuf);
     int32_t *parent = want_parent ? bp<int32_t>(pbuf) : nullptr;
     const double divisor = o.switch_divisor < 0 ? g->bfs_divisor : o.switch_divisor;
+    const double threshold = divisor > 0 ? (double)g->m / divisor : 0.0;
+    const unsigned long long whole = threshold < 0x1p40 ? (unsigned long long)threshold : 1ull << 40;
     const uint32_t *first = in_adj ? bp<uint32_t>(g->first_in) : nullptr;
     BfsLoop a{bp<uint32_t>(g->csr.ptr), bp<uint32_t>(g->csr.col), in_adj ? bp<uint32_t>(in_adj->ptr) : nullptr,
               in_adj ? bp<uint32_t>(in_adj->col) : nullptr, first, first ? first + first_words(n) : nullptr,
-              bp<uint32_t>(g->out_deg), n, nw, root, o.direction, divisor > 0 ? (double)g->m / divisor : 0.0, level, parent,
+              bp<uint32_t>(g->out_deg), n, nw, root, o.direction, threshold, whole, level, parent,
               bits, bits + nw4, {bits + 2 * nw4, bits + 3 * nw4}, reinterpret_cast<uint4 *>(wk), st};
     const uint64_t want = (g->m + n) / EG_BFSL_SHARE + 1, most = (uint64_t)ctx->sm_count * EG_BFSL_B;
     void *args[] = {&a};

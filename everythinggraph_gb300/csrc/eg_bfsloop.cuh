@@ -11,6 +11,8 @@
 // words that other SMs write go through L1 where an old value is harmless (a
 // visited bit missed is settled by the claim's atomicOr): every barrier makes
 // the writes before it visible.
+// Runs of small push levels go through one CTA while the others wait at a
+// barrier (bfsl_small).
 //
 // What bounds it: on small graphs the barriers (1.2 us each on a part-filled
 // grid, 4 .. 5 us with 304 CTAs) and one chain of dependent loads per step, on
@@ -34,6 +36,7 @@
 // grid by the entries alone (3 CTAs) 1456 us, by both 59.
 #define EG_BFSL_SHARE 4096u
 #define EG_BFSL_ALONE 8    // 16-byte steps of a pull's list that one lane takes
+#define EG_BFSL_SMALL 1024u  // edges of a push that one CTA takes alone
 #define EG_NO_VERTEX 0xffffffffu
 
 namespace {
@@ -44,6 +47,9 @@ struct BfsLoopState {
     uint32_t count[3];          // vertices of the level reached
     uint32_t levels, pull_levels, err;
     unsigned long long reached, traversed;
+    // what consecutive small levels left behind (bfsl_small)
+    uint32_t s_count, s_levels;
+    unsigned long long s_deg, s_reached, s_traversed;
 };
 
 struct BfsLoop {
@@ -51,6 +57,7 @@ struct BfsLoop {
     uint32_t n, nw, root;
     int dirmode;
     double threshold;
+    unsigned long long whole;  // the threshold, rounded down (bfsl_small)
     int32_t *level, *parent;
     uint32_t *visited, *prev, *bm[2];
     uint4 *queue;
@@ -85,6 +92,150 @@ __device__ __forceinline__ void bfsl_add(BfsTally t, uint32_t *count, unsigned l
             atomicAdd(count, t.count);
             atomicAdd(deg, t.deg);
         }
+    }
+}
+
+// Shared memory of a CTA: a pull's lists and words, or the two frontiers of
+// bfsl_small.
+union BfsSmem {
+    struct {
+        uint32_t list[EG_BFSL_T / 32][160];
+        uint32_t found[EG_BFSL_T / 32][4];
+    } pull;
+    struct {
+        uint2 q[2][EG_BFSL_SMALL];  // list start, length; from the level's scan on: start - place, first place
+        uint32_t v[2][EG_BFSL_SMALL];
+        uint32_t n[3], e[3], warp[EG_BFSL_T / 32];
+    } small;
+};
+
+__device__ __forceinline__ bool bfsl_wants_pull(const BfsLoop &a, uint32_t count, unsigned long long fdeg) {
+    return a.dirmode == EG_BFS_PULL_ONLY ||
+           (a.dirmode == EG_BFS_AUTO && count + fdeg > a.whole);
+}
+
+// Push levels of at most EG_BFSL_SMALL edges, one after another in CTA 0 until
+// the frontier is empty, larger, or one for a pull, the frontier in shared
+// memory and block barriers between levels.  A level is one chain of three
+// loads (entry, claim, row); by the whole grid it takes a list pass and two grid
+// barriers.  A level of a path of 20,000 / 300,000 vertices: 6.1 / 7.2 us by the
+// grid, now 1.1 / 1.3 to 2.1; a search of a 200 x 200 mesh 3.1 -> 0.9 ms, 1000 x 1000
+// 22.4 -> 18.5.  A call of its own, and with whole-number compares, so that the
+// other directions keep their registers (RMAT n = 16.8M, m = 537M: 429 us a
+// search without this, 432 so, 438 inlined or with FP64 compares left out).
+template <bool PARENT>
+__device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel, uint32_t it, BfsSmem &sm) {
+    auto &m = sm.small;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t cnt = (uint32_t)(sel >> 32), E = (uint32_t)sel, c = 0, levels = 0, slot = 0;
+    unsigned long long reached = 0, traversed = 0;
+    for (uint32_t i = tid; i < cnt; i += EG_BFSL_T) {  // the list comes with its places
+        const uint4 q = __ldcg(a.queue + i);
+        m.q[0][i] = make_uint2(q.y, q.x);
+        m.v[0][i] = q.z;
+    }
+    if (tid < 3) m.n[tid] = m.e[tid] = 0;
+    __syncthreads();
+    for (;;) {
+        const uint2 *q = m.q[c];
+        // up to 32 vertices: an entry per lane, every warp alike
+        uint2 mine = make_uint2(0u, 0xffffffffu);
+        if (cnt <= 32 && lane < cnt) mine = q[lane];
+        if (cnt <= 32 && levels) {
+            const uint32_t len = lane < cnt ? mine.y : 0u;
+            uint32_t x = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(EG_FULL_MASK, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            if (lane < cnt) mine = make_uint2(mine.x - (x - len), x - len);
+        }
+        const int32_t next_level = (int32_t)(it + levels) + 2;
+        for (uint32_t x0 = warp * 32; x0 < E; x0 += EG_BFSL_T) {
+            const uint32_t x = x0 + lane;
+            uint32_t o = 0, add;  // the last entry that begins at or before place x
+            if (cnt <= 32) {
+#pragma unroll
+                for (uint32_t s = 16; s > 0; s >>= 1)
+                    if (__shfl_sync(EG_FULL_MASK, mine.y, o + s) <= x) o += s;
+                add = __shfl_sync(EG_FULL_MASK, mine.x, o);
+            } else {
+                for (uint32_t hi = cnt; hi - o > 1;) {
+                    const uint32_t mid = (o + hi) >> 1;
+                    if (q[mid].y <= x) o = mid;
+                    else hi = mid;
+                }
+                add = q[o].x;
+            }
+            uint32_t v = 0, old = EG_FULL_MASK, bit = 0, start = 0, len = 0;
+            if (x < E) {
+                v = __ldg(a.col + (x + add));
+                bit = 1u << (v & 31);
+                old = atomicOr(a.visited + (v >> 5), bit);
+            }
+            const bool claimed = !(old & bit) && x < E;
+            if (claimed) {
+                start = __ldg(a.ptr + v);
+                len = __ldg(a.ptr + v + 1) - start;
+                a.level[v] = next_level;
+                if (PARENT) a.parent[v] = (int32_t)m.v[c][o];
+            }
+            const uint32_t ball = __ballot_sync(EG_FULL_MASK, claimed);
+            if (!ball) continue;
+            const uint32_t sum = __reduce_add_sync(EG_FULL_MASK, len);  // < 2^32 over all vertices
+            uint32_t at = 0;
+            if (lane == 0) {
+                at = atomicAdd(&m.n[slot], (uint32_t)__popc(ball));
+                atomicAdd(&m.e[slot], sum);
+            }
+            at = __shfl_sync(EG_FULL_MASK, at, 0) + __popc(ball & eg_lanemask_lt());
+            if (claimed) {
+                m.q[c ^ 1][at] = make_uint2(start, len);
+                m.v[c ^ 1][at] = v;
+            }
+        }
+        const uint32_t nslot = slot == 2 ? 0 : slot + 1;
+        if (tid == 0) m.n[nslot] = m.e[nslot] = 0;  // read before the last barrier, used after the next
+        __syncthreads();
+        cnt = m.n[slot];
+        E = m.e[slot];
+        slot = nslot;
+        c ^= 1;
+        levels++;
+        reached += cnt;
+        traversed += E;
+        if (!cnt || E > EG_BFSL_SMALL || bfsl_wants_pull(a, cnt, E) || it + levels > a.n) break;
+        // the frontier goes on here: visited & ~prev is to be what comes after it
+        for (uint32_t i = tid; i < cnt; i += EG_BFSL_T) {
+            const uint32_t v = m.v[c][i];
+            atomicOr(a.prev + (v >> 5), 1u << (v & 31));
+        }
+        if (cnt > 32) {  // places: two entries per thread
+            const uint32_t i = 2 * tid;
+            const uint2 q0 = i < cnt ? m.q[c][i] : make_uint2(0u, 0u), q1 = i + 1 < cnt ? m.q[c][i + 1] : make_uint2(0u, 0u);
+            const uint32_t s = q0.y + q1.y;
+            uint32_t x = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(EG_FULL_MASK, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            if (lane == 31) m.warp[warp] = x;
+            __syncthreads();
+            uint32_t off = x - s;
+            for (uint32_t w = 0; w < warp; w++) off += m.warp[w];
+            if (i < cnt) m.q[c][i] = make_uint2(q0.x - off, off);
+            if (i + 1 < cnt) m.q[c][i + 1] = make_uint2(q1.x - (off + q0.y), off + q0.y);
+            __syncthreads();
+        }
+    }
+    if (tid == 0) {
+        a.st->s_count = cnt;
+        a.st->s_levels = levels;
+        a.st->s_deg = E;
+        a.st->s_reached = reached;
+        a.st->s_traversed = traversed;
     }
 }
 
@@ -195,12 +346,10 @@ __device__ __forceinline__ uint32_t bfsl_scan(const BfsLoop &a, const uint32_t *
 // (scanned turn by turn: 412 us instead of 385 on the largest graph above).
 template <bool PARENT>
 __device__ __forceinline__ BfsTally bfsl_pull(const BfsLoop &a, const uint32_t *cur, uint32_t *next,
-                                              int32_t next_level) {
-    __shared__ uint32_t s_list[EG_BFSL_T / 32][160];
-    __shared__ uint32_t s_found[EG_BFSL_T / 32][4];
+                                              int32_t next_level, BfsSmem &sm) {
     BfsTally tally = {0u, 0ull};
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mine = lane >> 3, shift = 4 * (lane & 7);
-    uint32_t *list = s_list[warp], *found = s_found[warp];
+    uint32_t *list = sm.pull.list[warp], *found = sm.pull.found[warp];
     const uint32_t step = ((gridDim.x * blockDim.x) >> 5) * 4;
     uint32_t w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4, held = 0;
     uint32_t ahead = w0 + mine < a.nw ? __ldcg(a.visited + w0 + mine) : EG_FULL_MASK;
@@ -403,6 +552,7 @@ __device__ __forceinline__ void bfsl_list(const BfsLoop &a, unsigned long long *
 
 template <bool PARENT>
 __global__ void __launch_bounds__(EG_BFSL_T, EG_BFSL_B) k_bfs_loop(const BfsLoop a) {
+    __shared__ BfsSmem sm;
     auto grid = cooperative_groups::this_grid();
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     const uint32_t root = a.root;
@@ -434,7 +584,7 @@ __global__ void __launch_bounds__(EG_BFSL_T, EG_BFSL_B) k_bfs_loop(const BfsLoop
     }
     grid.sync();
     unsigned long long fdeg = d0, reached = 1, traversed = d0, sel = d0 ? (1ull << 32) | d0 : 0ull;
-    uint32_t count = 1, pulls = 0, set = 0, it = 0;
+    uint32_t count = 1, pulls = 0, set = 0, it = 0, lists = 0;
     int cur = 0;
     auto wants_pull = [&]() {
         return a.dirmode == EG_BFS_PULL_ONLY ||
@@ -446,34 +596,46 @@ __global__ void __launch_bounds__(EG_BFSL_T, EG_BFSL_B) k_bfs_loop(const BfsLoop
         if (i0 == 0) {  // no CTA reads these any more, and none adds to them yet
             a.st->deg[nset] = 0;
             a.st->count[nset] = 0;
-            a.st->sel[(it + 1) & 1] = 0;
+            a.st->sel[lists & 1] = 0;
         }
-        const int32_t next_level = (int32_t)it + 2;
-        const BfsTally t = pull ? bfsl_pull<PARENT>(a, a.bm[cur], a.bm[cur ^ 1], next_level)
-                                : bfsl_push<PARENT>(a, sel, next_level);
-        __syncwarp();
-        bfsl_add(t, &a.st->count[set], &a.st->deg[set]);
-        grid.sync();
-        count = __ldcg(&a.st->count[set]);
-        fdeg = __ldcg(&a.st->deg[set]);
-        reached += count;
-        traversed += fdeg;
-        pulls += pull;
+        const bool small = !pull && (uint32_t)(sel >> 32) <= EG_BFSL_SMALL && (uint32_t)sel <= EG_BFSL_SMALL;
+        if (small) {
+            if (blockIdx.x == 0) bfsl_small<PARENT>(a, sel, it, sm);
+            grid.sync();
+            count = __ldcg(&a.st->s_count);
+            fdeg = __ldcg(&a.st->s_deg);
+            reached += __ldcg(&a.st->s_reached);
+            traversed += __ldcg(&a.st->s_traversed);
+            it += __ldcg(&a.st->s_levels) - 1;
+        } else {
+            const int32_t next_level = (int32_t)it + 2;
+            const BfsTally t = pull ? bfsl_pull<PARENT>(a, a.bm[cur], a.bm[cur ^ 1], next_level, sm)
+                                    : bfsl_push<PARENT>(a, sel, next_level);
+            __syncwarp();
+            bfsl_add(t, &a.st->count[set], &a.st->deg[set]);
+            grid.sync();
+            count = __ldcg(&a.st->count[set]);
+            fdeg = __ldcg(&a.st->deg[set]);
+            reached += count;
+            traversed += fdeg;
+            pulls += pull;
+            set = nset;
+        }
         over = it > a.n;
         if (!count || over) break;
         const bool was = pull;
         pull = wants_pull();
         if (!pull) {
-            bfsl_list(a, &a.st->sel[(it + 1) & 1]);
+            bfsl_list(a, &a.st->sel[lists & 1]);
             grid.sync();
-            sel = __ldcg(&a.st->sel[(it + 1) & 1]);
+            sel = __ldcg(&a.st->sel[lists & 1]);
+            lists++;
         } else if (was) {
             cur ^= 1;
         } else {
             bfsl_bitmap(a, a.bm[cur]);
             grid.sync();
         }
-        set = nset;
     }
     if (i0 == 0) {
         a.st->levels = it + 1;
