@@ -149,6 +149,7 @@ static int bfs_core(eg_graph *g, uint32_t root, const eg_bfs_opts &o, int slot, 
         stats->reached = (uint32_t)h->reached;
         stats->edges_traversed = h->traversed;
         stats->pull_levels = (int)h->pull_levels;
+        EG_CUDA(cudaEventSynchronize(ctx->ev1));  // the flag may be seen before the event's completion
         EG_CUDA(cudaEventElapsedTime(&stats->ms, ctx->ev0, ctx->ev1));
     }
     return EG_OK;
