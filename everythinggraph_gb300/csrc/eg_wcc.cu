@@ -169,9 +169,34 @@ __global__ void __launch_bounds__(256) k_wcc_rest(const uint32_t *__restrict__ p
     }
 }
 
-// Every vertex's root into par and root, four vertices per thread, the parents
-// read through L1 (the low ids are most vertices' ancestors; an old line holds
-// an ancestor too).
+// The roots of vertices v .. v + 3 from their ancestors p.  The first
+// EG_WCC_HOPS steps read the parents through L1 (the low ids are most vertices'
+// ancestors; an old line holds an ancestor too).  Where they do not end, each
+// step is written to the vertices' own parents and read past L1, so that the
+// steps double: a forest of depth d takes EG_WCC_HOPS + log2(d) steps in place
+// of d (ids in order along a path: the seeds make one chain of it).
+#define EG_WCC_HOPS 6
+__device__ __forceinline__ void wcc_roots(uint32_t *par, uint32_t n, uint32_t v, uint32_t (&p)[4]) {
+    for (int hop = 0;; hop++) {  // parents only ever decrease: a stale one is still an ancestor
+        uint32_t g[4];
+        bool more = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++) g[i] = hop < EG_WCC_HOPS ? __ldca(par + p[i]) : __ldcg(par + p[i]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            more |= g[i] != p[i];
+            p[i] = g[i];
+        }
+        if (!more) break;
+        if (hop >= EG_WCC_HOPS) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (v + i < n) __stcg(par + v + i, p[i]);
+        }
+    }
+}
+
+// Every vertex's root into par and root, four vertices per thread.
 __global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, uint32_t *__restrict__ root) {
     const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
@@ -181,20 +206,9 @@ __global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, 
 #pragma unroll
         for (int i = 0; i < 4; i++)
             if (v + i >= n) p[i] = v;  // padding: any vertex
-        for (;;) {  // parents only ever decrease: a stale one is still an ancestor
-            uint32_t g[4];
-            bool more = false;
-#pragma unroll
-            for (int i = 0; i < 4; i++) g[i] = __ldca(par + p[i]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                more |= g[i] != p[i];
-                p[i] = g[i];
-            }
-            if (!more) break;
-        }
+        wcc_roots(par, n, v, p);
         const uint4 y = make_uint4(p[0], p[1], p[2], p[3]);
-        reinterpret_cast<uint4 *>(par)[q] = y;
+        if (y.x != x.x || y.y != x.y || y.z != x.z || y.w != x.w) reinterpret_cast<uint4 *>(par)[q] = y;
         reinterpret_cast<uint4 *>(root)[q] = y;
     }
 }
@@ -202,7 +216,7 @@ __global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, 
 // Every vertex's label: its root.  With a pick, root[] holds the roots from
 // before the last hooks: the vertices of the picked tree, mostly all, have
 // one label between them, found once per thread.  Counts the components.
-__global__ void __launch_bounds__(256) k_wcc_labels(uint32_t n, const uint32_t *par, uint32_t *label,
+__global__ void __launch_bounds__(256) k_wcc_labels(uint32_t n, uint32_t *par, uint32_t *label,
                                                     const WccPick *pick, unsigned long long *roots) {
     const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);
     const uint32_t skip = pick ? pick->root : EG_WCC_NONE;
@@ -219,21 +233,11 @@ __global__ void __launch_bounds__(256) k_wcc_labels(uint32_t n, const uint32_t *
             if (v + i >= n || p[i] == skip) p[i] = common;
             if (v + i >= n && skip == EG_WCC_NONE) p[i] = v;
         }
-        for (;;) {
-            uint32_t g[4];
-            bool more = false;
-#pragma unroll
-            for (int i = 0; i < 4; i++) g[i] = p[i] == common ? common : __ldca(par + p[i]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                more |= g[i] != p[i];
-                p[i] = g[i];
-            }
-            if (!more) break;
-        }
+        if (p[0] != common || p[1] != common || p[2] != common || p[3] != common) wcc_roots(par, n, v, p);
 #pragma unroll
         for (int i = 0; i < 4; i++) count += v + i < n && p[i] == v + i;
-        reinterpret_cast<uint4 *>(label)[q] = make_uint4(p[0], p[1], p[2], p[3]);
+        if (!pick || p[0] != x.x || p[1] != x.y || p[2] != x.z || p[3] != x.w)
+            reinterpret_cast<uint4 *>(label)[q] = make_uint4(p[0], p[1], p[2], p[3]);
     }
     count = __reduce_add_sync(EG_FULL_MASK, count);
     if ((threadIdx.x & 31) == 0 && count) atomicAdd(roots, (unsigned long long)count);
