@@ -70,27 +70,45 @@ struct WccPick {
 
 // par[v] = the least of v and the first entries of its lists (optr NULL: one
 // list); parents never exceed their children, so this is a forest.  Four
-// vertices per thread, their loads in flight together.
+// vertices per thread, their loads in flight together.  bits: a bit per vertex
+// with an edge.  Four vertices without one are done here: their root is
+// written, their parent nowhere read, and the passes that follow leave them out
+// by their bits (n = 16.8 M, 4 K entries: rest 61 us, flatten and labels 24 and
+// 28 us with row pointers and parents read; a call 174 -> 107).
 __global__ void __launch_bounds__(256) k_wcc_seed(const uint32_t *__restrict__ iptr, const uint32_t *__restrict__ icol,
                                                   const uint32_t *__restrict__ optr, const uint32_t *__restrict__ ocol,
-                                                  uint32_t n, uint32_t *__restrict__ par) {
-    const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const uint32_t v = 4 * q;
-        uint32_t p[4] = {v, v + 1, v + 2, v + 3};
-        for (int side = 0; side < 2; side++) {
+                                                  uint32_t n, uint32_t *__restrict__ par,
+                                                  uint32_t *__restrict__ root, uint32_t *__restrict__ bits) {
+    const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2), lane = threadIdx.x & 31;
+    // uniform trip count per warp
+    for (uint32_t q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); q0 < nq; q0 += gridDim.x * blockDim.x) {
+        const uint32_t q = q0 + lane, v = 4 * q;
+        uint32_t p[4] = {v, v + 1, v + 2, v + 3}, has = 0;
+        for (int side = 0; side < 2 && q < nq; side++) {
             const uint32_t *__restrict__ ptr = side ? optr : iptr, *__restrict__ col = side ? ocol : icol;
             if (!ptr) break;
             const uint4 r = __ldg(reinterpret_cast<const uint4 *>(ptr + v));  // past the end: the buffer's padding
             const uint32_t b[5] = {r.x, r.y, r.z, r.w, __ldg(ptr + v + 4)};
             uint32_t c[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) c[i] = v + i < n && b[i + 1] != b[i] ? __ldg(col + b[i]) : p[i];
+            for (int i = 0; i < 4; i++) {
+                const bool on = v + i < n && b[i + 1] != b[i];
+                c[i] = on ? __ldg(col + b[i]) : p[i];
+                has |= (uint32_t)on << i;
+            }
 #pragma unroll
             for (int i = 0; i < 4; i++) p[i] = c[i] < p[i] ? c[i] : p[i];
         }
-        reinterpret_cast<uint4 *>(par)[q] = make_uint4(p[0], p[1], p[2], p[3]);
+        if (q < nq) reinterpret_cast<uint4 *>(has ? par : root)[q] = make_uint4(p[0], p[1], p[2], p[3]);
+        uint32_t word = has << (4 * (lane & 7));
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) word |= __shfl_xor_sync(EG_FULL_MASK, word, o);
+        if (!(lane & 7) && q < nq) bits[q >> 3] = word;
     }
+}
+// Of the vertices 4 q .. 4 q + 3.
+__device__ __forceinline__ bool wcc_any_edge(const uint32_t *__restrict__ bits, uint32_t q) {
+    return (__ldg(bits + (q >> 3)) >> (4 * (q & 7))) & 15u;
 }
 
 // Roots of 512 sampled vertices with an edge (the first of four draws that
@@ -127,10 +145,12 @@ __global__ void __launch_bounds__(512) k_wcc_pick(const uint32_t *__restrict__ p
 
 // One round: root[] are the flattened roots, par[] is theirs on entry.
 __global__ void __launch_bounds__(256) k_wcc_round(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
-                                                   const uint32_t *__restrict__ root, uint32_t n, WccPick *pick,
+                                                   const uint32_t *__restrict__ root,
+                                                   const uint32_t *__restrict__ bits, uint32_t n, WccPick *pick,
                                                    uint32_t *par) {
     uint32_t hooks = 0;
     for (uint64_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
+        if (!((__ldg(bits + (u >> 5)) >> (u & 31)) & 1u)) continue;
         const uint32_t ru = __ldg(root + u), b = __ldg(ptr + u), d = __ldg(ptr + u + 1) - b;
         uint32_t rw[4];
 #pragma unroll
@@ -151,14 +171,17 @@ __global__ void __launch_bounds__(256) k_wcc_round(const uint32_t *__restrict__ 
 // (root[]: the roots before this kernel): a warp walks the lists of 32
 // vertices together.
 __global__ void __launch_bounds__(256) k_wcc_rest(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
-                                                  const uint32_t *__restrict__ root, uint32_t n,
+                                                  const uint32_t *__restrict__ root,
+                                                  const uint32_t *__restrict__ bits, uint32_t n,
                                                   const WccPick *__restrict__ pick, uint32_t *par) {
     const uint32_t skip = pick->root, lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint64_t v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); v0 < n; v0 += stride) {
         const uint32_t u = (uint32_t)v0 + lane;
+        const uint32_t on = __ldg(bits + (v0 >> 5));
+        if (!on) continue;
         uint32_t b = 0, d = 0;
-        if (v0 + lane < n && __ldg(root + u) != skip) {
+        if (((on >> lane) & 1u) && __ldg(root + u) != skip) {
             b = __ldg(ptr + u);
             d = __ldg(ptr + u + 1) - b;
         }
@@ -197,9 +220,11 @@ __device__ __forceinline__ void wcc_roots(uint32_t *par, uint32_t n, uint32_t v,
 }
 
 // Every vertex's root into par and root, four vertices per thread.
-__global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, uint32_t *__restrict__ root) {
+__global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, uint32_t *__restrict__ root,
+                                                     const uint32_t *__restrict__ bits) {
     const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+        if (!wcc_any_edge(bits, q)) continue;
         const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(par) + q);
         const uint32_t v = 4 * q;
         uint32_t p[4] = {x.x, x.y, x.z, x.w};
@@ -217,7 +242,8 @@ __global__ void __launch_bounds__(256) k_wcc_flatten(uint32_t n, uint32_t *par, 
 // before the last hooks: the vertices of the picked tree, mostly all, have
 // one label between them, found once per thread.  Counts the components.
 __global__ void __launch_bounds__(256) k_wcc_labels(uint32_t n, uint32_t *par, uint32_t *label,
-                                                    const WccPick *pick, unsigned long long *roots) {
+                                                    const WccPick *pick, const uint32_t *__restrict__ bits,
+                                                    unsigned long long *roots) {
     const uint32_t nq = (uint32_t)(((uint64_t)n + 3) >> 2);
     const uint32_t skip = pick ? pick->root : EG_WCC_NONE;
     uint32_t common = skip;
@@ -226,6 +252,10 @@ __global__ void __launch_bounds__(256) k_wcc_labels(uint32_t n, uint32_t *par, u
     uint32_t count = 0;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const uint32_t v = 4 * q;
+        if (pick && !wcc_any_edge(bits, q)) {
+            count += n - v < 4 ? n - v : 4;
+            continue;
+        }
         const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(pick ? label : par) + q);
         uint32_t p[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -281,12 +311,12 @@ extern "C" int eg_wcc(eg_graph *g, int64_t *labels_out, eg_wcc_stats *stats) {
     EG_CUDA(cudaSetDevice(ctx->device));
     const uint32_t n = g->n;
     EG_TRY(eg_buf_ensure(ctx, g->label, (uint64_t)n * 4));  // padded: written four vertices at a time
-    // work: parent[n] | counters | int64 staging for the host copy
-    const uint64_t off_cnt = ((uint64_t)n + 3) & ~3ull;
-    const uint64_t off_wide = off_cnt + 8;
+    // work: parent[n] | counters | a bit per vertex | int64 staging for the host copy
+    const uint64_t off_cnt = ((uint64_t)n + 3) & ~3ull, off_bits = off_cnt + 8;
+    const uint64_t off_wide = off_bits + (((uint64_t)n + 127) / 128) * 4;
     EG_TRY(eg_buf_ensure(ctx, g->bfs_work, (off_wide + (labels_out ? 2ull * n : 0)) * 4));
     uint32_t *par = bp<uint32_t>(g->bfs_work);
-    uint32_t *retries = par + off_cnt;
+    uint32_t *retries = par + off_cnt, *bits = par + off_bits;
     unsigned long long *roots = reinterpret_cast<unsigned long long *>(par + off_cnt + 2);
     long long *wide = reinterpret_cast<long long *>(par + off_wide);
     uint32_t blocks = (uint32_t)(ctx->sm_count * 8);
@@ -304,29 +334,32 @@ extern "C" int eg_wcc(eg_graph *g, int64_t *labels_out, eg_wcc_stats *stats) {
         const uint32_t *optr = sym ? nullptr : bp<uint32_t>(g->csr.ptr), *ocol = sym ? nullptr : bp<uint32_t>(g->csr.col);
         WccPick *pick = reinterpret_cast<WccPick *>(par + off_cnt + 4);
         uint32_t *root = bp<uint32_t>(g->label);
-        k_wcc_seed<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, optr, ocol, n, par);
+        k_wcc_seed<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, optr, ocol, n, par, root, bits);
         EG_LAUNCHED(ctx);
         WccPick *hp = reinterpret_cast<WccPick *>(ctx->h_pinned);
         for (int r = 0;; r++) {
-            k_wcc_flatten<<<blocks, 256, 0, ctx->stream>>>(n, par, root);
+            k_wcc_flatten<<<blocks, 256, 0, ctx->stream>>>(n, par, root, bits);
             EG_LAUNCHED(ctx);
             k_wcc_pick<<<1, 512, 0, ctx->stream>>>(par, iptr, optr, n, pick);
             EG_LAUNCHED(ctx);
             EG_TRY(eg_readback_wait(ctx, hp, pick, sizeof(WccPick), ctx->stream));
-            // most vertices in one tree, or a round that hooked next to nothing
-            if (r == EG_WCC_ROUNDS || 8ull * hp->count >= 7ull * hp->total || (r && hp->hooks < n / 256)) break;
+            // most vertices in one tree, or a round that hooked next to nothing,
+            // or entries so few that a round costs more than their finds
+            if (r == EG_WCC_ROUNDS || 8ull * hp->count >= 7ull * hp->total || (r && hp->hooks < n / 256) ||
+                g->m < n / 64)
+                break;
             EG_TRY(eg_zero(ctx, &pick->hooks, 4, ctx->stream));
-            k_wcc_round<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, root, n, pick, par);
+            k_wcc_round<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, root, bits, n, pick, par);
             EG_LAUNCHED(ctx);
             if (!sym) {
-                k_wcc_round<<<blocks, 256, 0, ctx->stream>>>(optr, ocol, root, n, pick, par);
+                k_wcc_round<<<blocks, 256, 0, ctx->stream>>>(optr, ocol, root, bits, n, pick, par);
                 EG_LAUNCHED(ctx);
             }
         }
-        k_wcc_rest<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, root, n, pick, par);
+        k_wcc_rest<<<blocks, 256, 0, ctx->stream>>>(iptr, icol, root, bits, n, pick, par);
         EG_LAUNCHED(ctx);
         if (!sym) {
-            k_wcc_rest<<<blocks, 256, 0, ctx->stream>>>(optr, ocol, root, n, pick, par);
+            k_wcc_rest<<<blocks, 256, 0, ctx->stream>>>(optr, ocol, root, bits, n, pick, par);
             EG_LAUNCHED(ctx);
         }
         picked = pick;
@@ -339,7 +372,7 @@ extern "C" int eg_wcc(eg_graph *g, int64_t *labels_out, eg_wcc_stats *stats) {
             EG_LAUNCHED(ctx);
         }
     }
-    k_wcc_labels<<<blocks, 256, 0, ctx->stream>>>(n, par, bp<uint32_t>(g->label), picked, roots);
+    k_wcc_labels<<<blocks, 256, 0, ctx->stream>>>(n, par, bp<uint32_t>(g->label), picked, bits, roots);
     EG_LAUNCHED(ctx);
     EG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     if (labels_out) {

@@ -51,3 +51,15 @@ def test_pagerank(n, tolerance):
     ctx.close()
     print(t)
     assert t[0] <= t[1], t
+
+
+def test_wcc():
+    ctx = __import__("everythinggraph_gb300").Context(0)
+    t = []
+    for m in (4096, None):
+        g = graph(ctx, 1 << 24, m)
+        t.append(best(lambda: g.wcc(copy_out=False)))
+        g.free()
+    ctx.close()
+    print(t)
+    assert t[0] <= t[1], t
