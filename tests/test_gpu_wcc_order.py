@@ -60,3 +60,21 @@ def test_time_of_a_path(n):
     ctx.close()
     print(t)
     assert t[0] <= 1.5 * t[1], t
+
+
+def test_time_of_a_path_through_shuffled_ids():
+    import everythinggraph_gb300 as eg
+
+    n = 1000000
+    rng = np.random.default_rng(1)
+    p = rng.permutation(n)
+    ctx = eg.Context(0)
+    t = []
+    for pairs in (np.stack([p[:-1], p[1:]], 1), rng.integers(0, n, (n, 2))):
+        g = ctx.from_pairs(n, pairs.astype(np.uint32).reshape(-1), undirected=True).build()
+        g.wcc(copy_out=False)
+        t.append(min(g.wcc(copy_out=False)[1].ms for _ in range(7)))
+        g.free()
+    ctx.close()
+    print(t)
+    assert t[0] <= 2.5 * t[1], t
