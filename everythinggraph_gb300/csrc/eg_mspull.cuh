@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_msp_light(const uint32_t *__restrict__ 
                 const uint32_t b = ptr[v], e = ptr[v + 1];
                 const uint32_t lim = e - b > EG_MSP_LIGHT ? b + EG_MSP_LIGHT : e;
                 uint32_t p = b;
-                for (; p + 4 <= lim; p += 4) {
+                for (const uint32_t whole = b + ((lim - b) & ~3u); p != whole; p += 4) {
                     const uint32_t u0 = col[p], u1 = col[p + 1], u2 = col[p + 2], u3 = col[p + 3];
                     acc |= (__ldg(front + u0) | __ldg(front + u1)) | (__ldg(front + u2) | __ldg(front + u3));
                     if ((acc & need) == need) break;
@@ -87,17 +87,16 @@ __global__ void __launch_bounds__(256) k_msp_mid(const uint32_t *__restrict__ pt
         unsigned long long tot = next[v];  // the light scan's partial word
         const uint32_t b = ptr[v] + EG_MSP_LIGHT, e = ptr[v + 1];
         const uint32_t lim = e - b > EG_MSP_MID ? b + EG_MSP_MID : e;
-        for (uint32_t base = b; base < lim; base += 128u) {
+        const uint32_t *__restrict__ c = col + b + lane;
+        for (uint32_t left = lim - b;; left -= 128u, c += 128) {  // entries left: places may not fit 32 bits
             unsigned long long acc = 0ull;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-                const uint32_t p = base + k * 32u + lane;
-                if (p < lim) acc |= __ldg(front + col[p]);
-            }
+            for (uint32_t k = 0; k < 4; k++)
+                if (left > k * 32u + lane) acc |= __ldg(front + c[k * 32u]);
             const uint32_t lo = __reduce_or_sync(EG_FULL_MASK, (uint32_t)acc);
             const uint32_t hi = __reduce_or_sync(EG_FULL_MASK, (uint32_t)(acc >> 32));
             tot |= ((unsigned long long)hi << 32) | lo;
-            if ((tot & need) == need) break;
+            if ((tot & need) == need || left <= 128u) break;
         }
         const bool more = (tot & need) != need && lim < e;
         if (lane == 0) {
@@ -123,18 +122,16 @@ __global__ void __launch_bounds__(256) k_msp_heavy(const uint32_t *__restrict__ 
         if (threadIdx.x == 0) s_acc = next[v];  // the earlier scans' partial word
         __syncthreads();
         const uint32_t e = ptr[v + 1];
-        for (uint32_t base = ptr[v] + EG_MSP_LIGHT + EG_MSP_MID; base < e; base += 1024u) {
+        for (uint32_t base = ptr[v] + EG_MSP_LIGHT + EG_MSP_MID;; base += 1024u) {  // below e
             unsigned long long acc = 0ull;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-                const uint32_t p = base + k * 256u + threadIdx.x;
-                if (p < e) acc |= __ldg(front + col[p]);
-            }
+            for (uint32_t k = 0; k < 4; k++)
+                if (e - base > k * 256u + threadIdx.x) acc |= __ldg(front + col[base + k * 256u + threadIdx.x]);
             const uint32_t lo = __reduce_or_sync(EG_FULL_MASK, (uint32_t)acc);
             const uint32_t hi = __reduce_or_sync(EG_FULL_MASK, (uint32_t)(acc >> 32));
             if (lane == 0 && (lo | hi)) atomicOr(&s_acc, ((unsigned long long)hi << 32) | lo);
             __syncthreads();
-            const bool stop = (s_acc & need) == need;
+            const bool stop = (s_acc & need) == need || e - base <= 1024u;
             __syncthreads();  // every thread has read s_acc before the next step adds to it
             if (stop) break;
         }

@@ -67,3 +67,35 @@ def test_sssp_round_over_all_entries():
     assert np.array_equal(dist, ref)
     assert st.relaxations == m
     ctx.close()
+
+
+@pytest.mark.parametrize("last", [33, 900, 3000])
+def test_multi_bfs_pull_of_the_last_list(last):
+    """The last vertex's in-list ends at entry 2^32 - 2 and has no reached
+    vertex: the pull reads it to the end and no further."""
+    import torch
+
+    import everythinggraph_gb300 as eg
+
+    need(190)
+    n, m = 40, 2 ** 32 - 2
+    pairs = torch.empty((m, 2), dtype=torch.int32, device="cuda")
+    pairs[:, 0] = 1
+    pairs[:, 1] = 3
+    pairs[-last:, 0] = 2
+    pairs[-last:, 1] = n - 1
+    pairs[-last - 1, 0], pairs[-last - 1, 1] = 3, 7
+    torch.cuda.synchronize()
+    ctx = eg.Context(0)
+    g = ctx.from_device_pairs(n, pairs.data_ptr(), m)
+    ctx.sync()
+    del pairs
+    torch.cuda.empty_cache()
+    g.build(eg.CSR | eg.CSC)
+    lv, st = g.bfs_multi(np.array([1, 3], dtype=np.uint32))
+    ref = np.zeros((2, n), dtype=np.int32)
+    ref[0, [1, 3, 7]] = 1, 2, 3
+    ref[1, [3, 7]] = 1, 2
+    assert np.array_equal(lv, ref)
+    assert st.pull_levels >= 1
+    ctx.close()
