@@ -181,6 +181,11 @@ int eg_ppr_plan(eg_graph *g) {
         QTRY(eg_fail(EG_ECUDA, "personalised PageRank plan: %s", cudaGetErrorString(cudaGetLastError())));
 #undef QTRY
     cleanup();
+    // a captured sweep holds the last plan's buffers and counts
+    eg_bfs_graph &bg = g->ppg;
+    if (bg.exec) cudaGraphExecDestroy(bg.exec);
+    if (bg.graph) cudaGraphDestroy(bg.graph);
+    bg = eg_bfs_graph();
     g->ppr_nlong = nlong;
     g->ppr_nmulti = nmulti;
     g->ppr_nrows = nrows;
@@ -256,9 +261,10 @@ extern "C" int eg_ppr_multi(eg_graph *g, const uint32_t *seeds, const uint32_t *
     EG_LAUNCHED(ctx);
     uint32_t dmg;
     memcpy(&dmg, &o.damping, 4);
-    // n and m are the graph's own; the seed offsets' place follows the seed count
-    const void *key[8] = {W, g->csc.col.p, (const void *)((uintptr_t)g->ppr_order.p ^ ((uintptr_t)g->ppr_long.p << 1)), (const void *)(uintptr_t)nq,
-                          (const void *)(uintptr_t)dmg, d_soff, g->csc.ptr.p, g->out_deg.p};
+    // n and m are the graph's own, a new plan drops the capture; the seed
+    // offsets' place follows the seed count
+    const void *key[8] = {W, g->csc.col.p, nullptr, (const void *)(uintptr_t)nq, (const void *)(uintptr_t)dmg, d_soff,
+                          g->csc.ptr.p, g->out_deg.p};
     eg_bfs_graph &bg = g->ppg;
     bool same = bg.exec != nullptr;
     for (int i = 0; i < 8 && same; i++) same = bg.key[i] == key[i];

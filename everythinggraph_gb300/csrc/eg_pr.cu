@@ -372,7 +372,7 @@ static int coo_launch(eg_graph *g, eg_adj &adj, eg_buf &carry_buf, eg_sum2 *part
         EG_ROW_TILE(128, 0)
         EG_ROW_TILE(256, 1)
     }
-        if constexpr (SPMV || (MK && !REDUCE)) {
+    if constexpr (SPMV || (MK && !REDUCE)) {
         EG_ROW_TILE(512, 1)
     }
     return coo_launch_t<Op, 1024, 4, REDUCE, 1, 5, H, MK>(g, adj, carry_buf, part, op, nparts, ev_begin, ev_end,

@@ -26,3 +26,21 @@ def test_row_of_equal_entries(length, extra):
     adds = 7 + min(-(-length // 8), 64) + (7 + -(-parts // 32) + 3 if parts > 1 else 0)
     assert abs(float(rank[0, 0]) - exact) <= (adds + 3) * 2.0 ** -24 * exact
     ctx.close()
+
+
+def test_after_loading_layouts(tmp_path):
+    """Layouts loaded into a graph that has run: the same queries, the same
+    bits."""
+    import everythinggraph_gb300 as eg
+
+    ctx = eg.Context(0)
+    g = ctx.rmat(14, 1 << 18, 3, undirected=True).build(eg.CSR | eg.CSC)
+    seeds = [[int(s)] for s in g.sample_roots(5, 1)]
+    ref, _ = g.ppr(seeds)
+    path = str(tmp_path / "g.eglayout")
+    g.save_layouts(path)
+    for _ in range(2):
+        assert g.load_layouts(path)
+        rank, _ = g.ppr(seeds)
+        assert np.array_equal(rank.view(np.uint32), ref.view(np.uint32))
+    ctx.close()
