@@ -95,16 +95,18 @@ __device__ __forceinline__ void bfsl_add(BfsTally t, uint32_t *count, unsigned l
     }
 }
 
-// Shared memory of a CTA: a pull's lists and words, or the two frontiers of
-// bfsl_small.
+// Shared memory of a CTA: a pull's lists and words, or the frontier of
+// bfsl_small.  13 KB with the rest: two CTAs leave 196 KB of the SM to L1, which
+// the pulls read their bitmaps through (25 KB: 164, pull-only searches of uniform
+// n = 1M, m = 16M 297 -> 377 us).
 union BfsSmem {
     struct {
         uint32_t list[EG_BFSL_T / 32][160];
         uint32_t found[EG_BFSL_T / 32][4];
     } pull;
     struct {
-        uint2 q[2][EG_BFSL_SMALL];  // list start, length; from the level's scan on: start - place, first place
-        uint32_t v[2][EG_BFSL_SMALL];
+        uint2 q[EG_BFSL_SMALL];  // list start, length; from the level's scan on: start - place, first place
+        uint32_t v[EG_BFSL_SMALL];
         uint32_t n[3], e[3], warp[EG_BFSL_T / 32];
     } small;
 };
@@ -119,28 +121,28 @@ __device__ __forceinline__ bool bfsl_wants_pull(const BfsLoop &a, uint32_t count
 // memory and block barriers between levels.  A level is one chain of three
 // loads (entry, claim, row); by the whole grid it takes a list pass and two grid
 // barriers.  A level of a path of 20,000 / 300,000 vertices: 6.1 / 7.2 us by the
-// grid, now 1.1 / 1.3 to 2.1; a search of a 200 x 200 mesh 3.1 -> 0.9 ms, 1000 x 1000
+// grid, now 1.4 / 2.1; a search of a 200 x 200 mesh 3.1 -> 1.0 ms, 1000 x 1000
 // 22.4 -> 18.5.  A call of its own, and with whole-number compares, so that the
-// other directions keep their registers (RMAT n = 16.8M, m = 537M: 429 us a
-// search without this, 432 so, 438 inlined or with FP64 compares left out).
+// other directions keep their registers (RMAT n = 16.8M, m = 537M: 430 us a
+// search without this, 432 so, 438 inlined).
 template <bool PARENT>
 __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel, uint32_t it, BfsSmem &sm) {
+    static_assert(EG_BFSL_SMALL == 2 * EG_BFSL_T, "two edges, and two entries, per thread");
     auto &m = sm.small;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t cnt = (uint32_t)(sel >> 32), E = (uint32_t)sel, c = 0, levels = 0, slot = 0;
+    uint32_t cnt = (uint32_t)(sel >> 32), E = (uint32_t)sel, levels = 0, slot = 0;
     unsigned long long reached = 0, traversed = 0;
     for (uint32_t i = tid; i < cnt; i += EG_BFSL_T) {  // the list comes with its places
         const uint4 q = __ldcg(a.queue + i);
-        m.q[0][i] = make_uint2(q.y, q.x);
-        m.v[0][i] = q.z;
+        m.q[i] = make_uint2(q.y, q.x);
+        m.v[i] = q.z;
     }
     if (tid < 3) m.n[tid] = m.e[tid] = 0;
     __syncthreads();
     for (;;) {
-        const uint2 *q = m.q[c];
         // up to 32 vertices: an entry per lane, every warp alike
         uint2 mine = make_uint2(0u, 0xffffffffu);
-        if (cnt <= 32 && lane < cnt) mine = q[lane];
+        if (cnt <= 32 && lane < cnt) mine = m.q[lane];
         if (cnt <= 32 && levels) {
             const uint32_t len = lane < cnt ? mine.y : 0u;
             uint32_t x = len;
@@ -152,8 +154,11 @@ __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel
             if (lane < cnt) mine = make_uint2(mine.x - (x - len), x - len);
         }
         const int32_t next_level = (int32_t)(it + levels) + 2;
-        for (uint32_t x0 = warp * 32; x0 < E; x0 += EG_BFSL_T) {
-            const uint32_t x = x0 + lane;
+        uint32_t at[2], u[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t x = tid + EG_BFSL_T * j;
+            if (warp * 32 + EG_BFSL_T * j >= E) break;
             uint32_t o = 0, add;  // the last entry that begins at or before place x
             if (cnt <= 32) {
 #pragma unroll
@@ -163,14 +168,22 @@ __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel
             } else {
                 for (uint32_t hi = cnt; hi - o > 1;) {
                     const uint32_t mid = (o + hi) >> 1;
-                    if (q[mid].y <= x) o = mid;
+                    if (m.q[mid].y <= x) o = mid;
                     else hi = mid;
                 }
-                add = q[o].x;
+                add = m.q[o].x;
             }
+            at[j] = x + add;
+            u[j] = PARENT ? m.v[o] : 0u;
+        }
+        __syncthreads();  // the frontier is read: the next one takes its place
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t x = tid + EG_BFSL_T * j;
+            if (warp * 32 + EG_BFSL_T * j >= E) break;
             uint32_t v = 0, old = EG_FULL_MASK, bit = 0, start = 0, len = 0;
             if (x < E) {
-                v = __ldg(a.col + (x + add));
+                v = __ldg(a.col + at[j]);
                 bit = 1u << (v & 31);
                 old = atomicOr(a.visited + (v >> 5), bit);
             }
@@ -179,20 +192,20 @@ __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel
                 start = __ldg(a.ptr + v);
                 len = __ldg(a.ptr + v + 1) - start;
                 a.level[v] = next_level;
-                if (PARENT) a.parent[v] = (int32_t)m.v[c][o];
+                if (PARENT) a.parent[v] = (int32_t)u[j];
             }
             const uint32_t ball = __ballot_sync(EG_FULL_MASK, claimed);
             if (!ball) continue;
             const uint32_t sum = __reduce_add_sync(EG_FULL_MASK, len);  // < 2^32 over all vertices
-            uint32_t at = 0;
+            uint32_t place = 0;
             if (lane == 0) {
-                at = atomicAdd(&m.n[slot], (uint32_t)__popc(ball));
+                place = atomicAdd(&m.n[slot], (uint32_t)__popc(ball));
                 atomicAdd(&m.e[slot], sum);
             }
-            at = __shfl_sync(EG_FULL_MASK, at, 0) + __popc(ball & eg_lanemask_lt());
+            place = __shfl_sync(EG_FULL_MASK, place, 0) + __popc(ball & eg_lanemask_lt());
             if (claimed) {
-                m.q[c ^ 1][at] = make_uint2(start, len);
-                m.v[c ^ 1][at] = v;
+                m.q[place] = make_uint2(start, len);
+                m.v[place] = v;
             }
         }
         const uint32_t nslot = slot == 2 ? 0 : slot + 1;
@@ -201,19 +214,18 @@ __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel
         cnt = m.n[slot];
         E = m.e[slot];
         slot = nslot;
-        c ^= 1;
         levels++;
         reached += cnt;
         traversed += E;
         if (!cnt || E > EG_BFSL_SMALL || bfsl_wants_pull(a, cnt, E) || it + levels > a.n) break;
         // the frontier goes on here: visited & ~prev is to be what comes after it
         for (uint32_t i = tid; i < cnt; i += EG_BFSL_T) {
-            const uint32_t v = m.v[c][i];
+            const uint32_t v = m.v[i];
             atomicOr(a.prev + (v >> 5), 1u << (v & 31));
         }
         if (cnt > 32) {  // places: two entries per thread
             const uint32_t i = 2 * tid;
-            const uint2 q0 = i < cnt ? m.q[c][i] : make_uint2(0u, 0u), q1 = i + 1 < cnt ? m.q[c][i + 1] : make_uint2(0u, 0u);
+            const uint2 q0 = i < cnt ? m.q[i] : make_uint2(0u, 0u), q1 = i + 1 < cnt ? m.q[i + 1] : make_uint2(0u, 0u);
             const uint32_t s = q0.y + q1.y;
             uint32_t x = s;
 #pragma unroll
@@ -225,8 +237,8 @@ __device__ __noinline__ void bfsl_small(const BfsLoop &a, unsigned long long sel
             __syncthreads();
             uint32_t off = x - s;
             for (uint32_t w = 0; w < warp; w++) off += m.warp[w];
-            if (i < cnt) m.q[c][i] = make_uint2(q0.x - off, off);
-            if (i + 1 < cnt) m.q[c][i + 1] = make_uint2(q1.x - (off + q0.y), off + q0.y);
+            if (i < cnt) m.q[i] = make_uint2(q0.x - off, off);
+            if (i + 1 < cnt) m.q[i + 1] = make_uint2(q1.x - (off + q0.y), off + q0.y);
             __syncthreads();
         }
     }
