@@ -377,7 +377,13 @@ __device__ __forceinline__ eg_sum3 eg_block_sum(eg_sum3 x, eg_sum2 *s_sum) {
     const uint32_t lane = threadIdx.x & 31;
     if (!(lane & 15)) (lane ? s_sum[threadIdx.x >> 5].b : s_sum[threadIdx.x >> 5].a) = x;
     __syncthreads();
-    if (threadIdx.x < 32) x = eg_warp_sum(lane < (blockDim.x >> 5) ? s_sum[lane] : eg_sum2());
+    if (threadIdx.x < 32) {  // two warps' words of the half's sum per lane
+        const uint32_t warps = blockDim.x >> 5, w = lane & 15;
+        const eg_sum3 *p = reinterpret_cast<const eg_sum3 *>(s_sum) + (lane >> 4);
+        x = w < warps ? p[2 * w] : eg_sum3();
+        if (w + 16 < warps) x.add(p[2 * (w + 16)]);
+        x = eg_half_sum(x);
+    }
     return x;
 }
 __device__ __forceinline__ eg_sum3 eg_block_sum(const eg_sum2 &acc, eg_sum2 *s_sum) {

@@ -70,6 +70,38 @@ __device__ __forceinline__ uint32_t prs_rows_below(const uint32_t *__restrict__ 
     return lo;
 }
 
+// The total of the CTAs' first (which 0) or second sums, in lane 0 of a warp,
+// all of a lane's loads in flight up to 160 CTAs; past fp32's range in FP64.
+__device__ __forceinline__ double prs_total(const eg_sum2 *part, uint32_t n, uint32_t which) {
+    const uint32_t lane = threadIdx.x & 31;
+    auto at = [&](uint32_t i) {
+        const float *p = reinterpret_cast<const float *>(part + i) + 3 * which;
+        eg_sum3 x;
+        if (i < n) {
+            x.s = __ldcg(p);
+            x.c = __ldcg(p + 1);
+            x.e = __ldcg(p + 2);
+        }
+        return x;
+    };
+    eg_sum3 sum;
+    for (uint32_t i = lane; i - lane < n; i += 160) {
+        eg_sum3 x[5];
+#pragma unroll
+        for (uint32_t k = 0; k < 5; k++) x[k] = at(i + 32 * k);
+#pragma unroll
+        for (uint32_t k = 0; k < 5; k++) sum.add(x[k]);
+    }
+    sum.add(eg_shfl_xor(sum, 16));
+    sum = eg_half_sum(sum);
+    if (__all_sync(EG_FULL_MASK, isfinite(sum.s))) return sum.wide();
+    double t = 0.0;
+    for (uint32_t i = lane; i < n; i += 32) t += at(i).wide();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(EG_FULL_MASK, t, o);
+    return t;
+}
+
 // REDUCE: the residual and the dangling mass are wanted (a tolerance, or
 // dangling mass spread).
 template <bool REDUCE, bool STAGE>
@@ -123,36 +155,29 @@ __global__ void __launch_bounds__(EG_PRS_THREADS, 1) k_pr_small(const PrSmall a)
         const float *cin = odd ? a.c1 : a.c0;
         float *cout = odd ? a.c0 : a.c1;
         // the sums of the last pass, by every CTA alike: the next base, the stop test
-        if (warp == 0) {
-            double2 t = make_double2(0.0, 0.0);
-            if (REDUCE) {
-                const eg_sum2 *part = a.part + (it & 1) * G;
-                eg_sum3 sum;
-                for (uint32_t i0 = lane & 15; i0 < G; i0 += 80) {  // five of a lane's loads in flight
-                    eg_sum3 x[5];
-#pragma unroll
-                    for (uint32_t k = 0; k < 5; k++) x[k] = eg_load_sum(part + i0 + 16 * k, i0 + 16 * k < G);
-#pragma unroll
-                    for (uint32_t k = 0; k < 5; k++) sum.add(x[k]);
-                }
-                t = eg_total(eg_half_sum(sum), part, G);
-            }
-            if (lane == 0) {
-                s_base = (float)(a.dangling ? a.base0 + a.per_dangling * t.y : a.base0);
-                s_done = it == a.iterations || (REDUCE && it && a.tol > 0.0 && t.x < a.tol);
+        if (warp < 2) {
+            // warp 0: the residual and the stop test, warp 1: the dangling mass and the base
+            double t = 0.0;
+            if (REDUCE) t = prs_total(a.part + (it & 1) * G, G, warp);
+            if (lane == 0 && warp == 0) {
+                s_done = it == a.iterations || (REDUCE && it && a.tol > 0.0 && t < a.tol);
                 if (b == 0 && s_done) {
-                    a.st->base = s_base;
                     a.st->done = it < a.iterations;
                     a.st->iters = it;
-                    a.st->residual = it ? t.x : 0.0;
-                    a.st->dangling = t.y;
+                    a.st->residual = it ? t : 0.0;
+                }
+            } else if (lane == 0) {
+                s_base = (float)(a.dangling ? a.base0 + a.per_dangling * t : a.base0);
+                if (b == 0) {  // the last pass's stay
+                    a.st->base = s_base;
+                    a.st->dangling = t;
                 }
             }
         } else if (STAGE && (it == 0 || a.swap)) {
             const uint32_t nq = a.n >> 2;
-            for (uint32_t i = tid - 32; i < nq; i += EG_PRS_THREADS - 32)
+            for (uint32_t i = tid - 64; i < nq; i += EG_PRS_THREADS - 64)
                 reinterpret_cast<float4 *>(s_c)[i] = __ldcg(reinterpret_cast<const float4 *>(cin) + i);
-            if (tid - 32 < (a.n & 3)) s_c[4 * nq + tid - 32] = __ldcg(cin + 4 * nq + tid - 32);
+            if (tid - 64 < (a.n & 3)) s_c[4 * nq + tid - 64] = __ldcg(cin + 4 * nq + tid - 64);
         }
         __syncthreads();
         if (s_done) break;
