@@ -146,8 +146,6 @@ def run_ours(args):
     g.tune()  # row schedule and BFS switch divisor for this graph (untimed setup)
     roots = g.sample_roots(W["roots"], W["root_seed"])
     stream = torch.cuda.ExternalStream(ctx.stream)
-    # host_loop as the caller asked (one level loop serves every value)
-    bfs_form = {"auto": None, "graph": False, "host": True}[args.bfs_form]
 
     # host outputs of the end-to-end step: page-locked, allocated once and
     # reused by every call (what a serving process holds); eg_bfs_batch takes
@@ -162,12 +160,11 @@ def run_ours(args):
         traversed = 0
         if copy_out:
             for c in range(0, len(roots), eb):
-                _, _, sts = g.bfs_batch(roots[c:c + eb], parents=True, level_out=lv_h, parent_out=par_h,
-                                        host_loop=bfs_form)
+                _, _, sts = g.bfs_batch(roots[c:c + eb], parents=True, level_out=lv_h, parent_out=par_h)
                 traversed += sum(st.edges_traversed for st in sts)
         else:
             for r in roots:
-                lv, par, st = g.bfs(int(r), parents=True, copy_out=False, host_loop=bfs_form)
+                lv, par, st = g.bfs(int(r), parents=True, copy_out=False)
                 traversed += st.edges_traversed
         lab, wst = g.wcc(copy_out=copy_out, out=lab_h)
         return traversed + m_in, traversed
@@ -648,23 +645,21 @@ def cache_report(ctx, eg, scale=24, path=None):
 
 
 def bfs_report(ctx, eg, scale=24, roots=16):
-    """Single-source BFS (levels + parents) on the undirected RMAT graph with
-    both values of host_loop (one level loop serves both), plus WCC."""
+    """Single-source BFS (levels + parents) on the undirected RMAT graph, plus WCC."""
     n = 1 << scale
     g = ctx.rmat(scale, 16 * n, 2, undirected=True).build(eg.CSR | eg.CSC)
     rs = g.sample_roots(roots, 3)
     out = {"workload": "bfs rmat%d undirected, %d roots" % (scale, roots)}
-    for name, host_loop in (("graph_loop", False), ("host_loop", True)):
-        g.bfs(int(rs[0]), parents=True, copy_out=False, host_loop=host_loop)
-        ms, te, lv, pl = 0.0, 0, 0, 0
-        for r in rs:
-            _, _, st = g.bfs(int(r), parents=True, copy_out=False, host_loop=host_loop)
-            ms += st.ms
-            te += st.edges_traversed
-            lv += st.levels
-            pl += st.pull_levels
-        out[name] = {"ms_per_bfs": ms / roots, "gteps": te / (ms / 1e3) / 1e9, "levels": lv / roots,
-                     "pull_levels": pl / roots}
+    g.bfs(int(rs[0]), parents=True, copy_out=False)
+    ms, te, lv, pl = 0.0, 0, 0, 0
+    for r in rs:
+        _, _, st = g.bfs(int(r), parents=True, copy_out=False)
+        ms += st.ms
+        te += st.edges_traversed
+        lv += st.levels
+        pl += st.pull_levels
+    out["bfs"] = {"ms_per_bfs": ms / roots, "gteps": te / (ms / 1e3) / 1e9, "levels": lv / roots,
+                  "pull_levels": pl / roots}
     g.wcc(copy_out=False)
     _, st = g.wcc(copy_out=False)
     out["wcc"] = {"ms": st.ms, "components": st.components, "rounds": st.rounds}
@@ -714,8 +709,6 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--scale", type=int, default=0)
     ap.add_argument("--no-extras", action="store_true")
-    ap.add_argument("--bfs-form", choices=["auto", "graph", "host"], default="auto",
-                    help="host_loop of the BFS calls (one level loop serves all three)")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--e2e-batch", type=int, default=E2E_BATCH, help="roots per eg_bfs_batch call in the end-to-end step")
     ap.add_argument("--pr-only", action="store_true", help="only the PageRank pull report (profiling)")

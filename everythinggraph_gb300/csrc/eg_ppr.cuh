@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256, EG_PPR_MINB) k_ppr_rows(const uint32_t *_
 // Rows in parts: a warp per row adds its part sums, group g the g-th quarter
 // of them in order with EG_PPR_FIXUP in flight, then the quarters in order.
 // (A hub has thousands of parts: one load per step made their chain of
-// latencies the kernel: undirected RMAT-20 64 us a sweep, now 12.)
+// latencies the kernel: undirected RMAT-20 64 us a sweep, now 8.)
 #define EG_PPR_FIXUP 8
 __global__ void __launch_bounds__(256) k_ppr_fixup(const uint4 *__restrict__ multi, uint32_t nmulti,
                                                    const float *__restrict__ part, float *__restrict__ Y) {
@@ -140,8 +140,12 @@ __global__ void __launch_bounds__(256) k_ppr_fixup(const uint4 *__restrict__ mul
         float4 x[EG_PPR_FIXUP];
 #pragma unroll
         for (uint32_t i = 0; i < EG_PPR_FIXUP; i++)
-            x[i] = k + i < k1 ? __ldcg(P4 + (uint64_t)(k + i) * (EG_PPR_LANES / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        acc = eg_f4add(acc, eg_f4sum8(x));
+            if (k + i < k1) x[i] = __ldcg(P4 + (uint64_t)(k + i) * (EG_PPR_LANES / 4));
+        float4 s = x[0];
+#pragma unroll
+        for (uint32_t i = 1; i < EG_PPR_FIXUP; i++)
+            if (k + i < k1) s = eg_f4add(s, x[i]);
+        acc = eg_f4add(acc, s);
     }
     float4 tot = eg_f4shfl(EG_FULL_MASK, acc, (int)sl);
 #pragma unroll
