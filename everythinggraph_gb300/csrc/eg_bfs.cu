@@ -32,7 +32,7 @@ __global__ void k_first_in(const uint32_t *__restrict__ ptr, const uint32_t *__r
     for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const uint32_t b = ptr[v], e = ptr[v + 1];
         unsigned long long best = 0ull;  // (degree << 32) | ~id: the max is the largest degree, then the smallest id
-        for (uint32_t p = b + lane; p < e; p += 32) {
+        for (uint64_t p = (uint64_t)b + lane; p < e; p += 32) {  // p + 32 may not fit 32 bits
             const uint32_t u = col[p];
             const unsigned long long key = ((unsigned long long)deg[u] << 32) | (uint32_t)~u;
             best = key > best ? key : best;

@@ -27,7 +27,7 @@ __device__ __forceinline__ void eg_warp_lists(uint32_t u, uint32_t b, uint32_t d
     }
     const uint32_t total = __shfl_sync(EG_FULL_MASK, inc, 31);
     const uint32_t exc = inc - d;
-    for (uint32_t p0 = 0; p0 < total; p0 += 32) {
+    for (uint32_t p0 = 0, left = total; left; p0 += 32, left = left > 32 ? left - 32 : 0) {
         const uint32_t x = p0 + lane;
         uint32_t lo = 0;  // owner of slot x: the first lane whose inclusive sum exceeds x
 #pragma unroll
@@ -38,7 +38,7 @@ __device__ __forceinline__ void eg_warp_lists(uint32_t u, uint32_t b, uint32_t d
         const uint32_t ob = __shfl_sync(EG_FULL_MASK, b, lo);
         const uint32_t oe = __shfl_sync(EG_FULL_MASK, exc, lo);
         const uint32_t ou = __shfl_sync(EG_FULL_MASK, u, lo);
-        const bool valid = x < total;
+        const bool valid = lane < left;  // x may not fit 32 bits
         f(valid, lo, ou, valid ? ob + (x - oe) : 0u);
     }
 }

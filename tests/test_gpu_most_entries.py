@@ -99,3 +99,39 @@ def test_multi_bfs_pull_of_the_last_list(last):
     assert np.array_equal(lv, ref)
     assert st.pull_levels >= 1
     ctx.close()
+
+
+def test_bfs_and_wcc_over_all_entries():
+    """Lists of about 4096 entries up to entry 2^32 - 2: all vertices within
+    three levels of any root, one component."""
+    import torch
+
+    import everythinggraph_gb300 as eg
+
+    need(190)
+    n, m = 1 << 20, 2 ** 32 - 2
+    ctx = eg.Context(0)
+    g = ctx.er(n, m, 11).build(eg.CSR | eg.CSC)
+    deg = g.degrees()[0].astype(np.int64)
+    start = np.concatenate([[0], np.cumsum(deg)])
+    assert start[-1] == m
+
+    class Col:
+        __cuda_array_interface__ = {"shape": (m,), "typestr": "<i4", "version": 3,
+                                    "data": (g.device_ptr(eg.L.EG_DEV_CSR_COL), False)}
+
+    col = torch.as_tensor(Col(), device="cuda")
+    for root in (n - 1, 12345):  # the first's list is the last one
+        near = np.unique(col[int(start[root]):int(start[root + 1])].cpu().numpy())
+        ref = np.full(n, 3, dtype=np.int32)
+        ref[near] = 2
+        ref[root] = 1
+        for direction in ("auto", "push", "pull"):
+            lv, par, st = g.bfs(root, direction=direction, parents=True)
+            assert np.array_equal(np.minimum(lv, 3), ref) and lv.max() <= 4
+            assert st.reached == n and st.edges_traversed == m
+            assert np.all(lv[par] == np.maximum(lv - 1, 1))
+    lab, st = g.wcc()
+    assert st.components == 1 and not lab.any()
+    del col
+    ctx.close()
